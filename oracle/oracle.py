@@ -36,7 +36,7 @@ def build(reference_root: str | None = REFERENCE_ROOT) -> None:
     """Compile the C restatement, and the reference solver when its sources exist
     (the reference source tree comes from $ANALOGSAT_REF, default /root/reference)."""
     subprocess.run(["make", "-s", "-C", HERE, "oracle"], check=True)
-    if reference_root and os.path.isdir(reference_root):
+    if reference_root and os.path.isdir(os.path.join(reference_root, "AnalogSAT")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "refcuda", f"REF={reference_root}"], check=True)
 
 
