@@ -23,6 +23,7 @@
 #include "as_kernels.cuh"
 #include "as_problem.h"
 #include "as_stream.cuh"
+#include "as_viol.cuh"
 
 using namespace asb;
 
@@ -725,13 +726,36 @@ int dispatch_rhs(as_problem* p, const T* x, T* d, int ns, void* stream) {
 
 template <typename T, int KMAX, bool EXACT>
 int launch_viol(as_problem* p, const T* x, int* c, int ns, cudaStream_t st) {
-    constexpr int BT = 256;
     constexpr int prec = sizeof(T) == 8 ? AS_PREC_F64 : AS_PREC_F32_LOGA;
-    const auto& q = p->packed(prec);
-    return launch_per_state<T, int>(p, prec, &viol_batch_kernel<T, KMAX, EXACT, BT, false>,
-                                    &viol_batch_kernel<T, KMAX, EXACT, BT, true>, BT,
-                                    (size_t)((q.n + 1 + 3) & ~3), q.compact, x, c, ns,
-                                    (long long)(q.n + q.m), st);
+    const DevInstance& I = p->dev[prec].host_inst[0];
+    const bool compact = I.lit != nullptr;
+    const long long stride = (long long)I.n + I.m;
+    int dev = 0, sms = 0;
+    AS_CUDA(cudaGetDevice(&dev));
+    AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (compact) {  // N < 32768: the masks fit one SM
+        const size_t smem = 4 * ((size_t)I.n + 1);
+        // States per group: as many as 32 while every SM still gets about four CTAs (so
+        // that the mask loads of one CTA overlap the clause checks of another), fewer for
+        // few states.  CTAs of a call with no more groups than SMs run alone on their
+        // SM and get all its threads.
+        const int resident = std::max(1, std::min(4, (int)(200 * 1024 / (smem + 1024))));
+        const int per = std::max(1, std::min(32, (ns + sms * resident - 1) / (sms * resident)));
+        const int grid = (ns + per - 1) / per;
+        auto fn = grid > sms ? &viol_group_kernel<T, KMAX, EXACT, 256> : &viol_group_kernel<T, KMAX, EXACT, 1024>;
+        if (smem > 47 * 1024) AS_CUDA(raise_smem_limit((const void*)fn, smem));
+        fn<<<grid, grid > sms ? 256 : 1024, smem, st>>>(I, x, c, ns, stride, per);
+    } else {
+        const int groups = (ns + 31) / 32, gy = std::min(groups, 65535);
+        AS_CUDA(p->slab[prec].alloc(4 * (size_t)groups * ((size_t)I.n + 1)));
+        uint32_t* gmask = p->slab[prec].template as<uint32_t>();
+        viol_mask_kernel<T><<<dim3((I.n + 256) / 256, gy), 256, 0, st>>>(I, x, c, gmask, ns, stride);
+        // about eight CTAs per SM over all groups, at least four clauses per thread
+        const int slices = std::max(1, std::min((I.m + 1023) / 1024, (8 * sms + gy - 1) / gy));
+        viol_count_kernel<KMAX, EXACT><<<dim3(slices, gy), 256, 0, st>>>(I, c, gmask, ns);
+    }
+    AS_CUDA(cudaGetLastError());
+    return AS_OK;
 }
 
 template <typename T>

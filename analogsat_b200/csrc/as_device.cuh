@@ -285,20 +285,6 @@ __device__ __forceinline__ int clause_violated(const DevInstance& I, int m, cons
     return sat ? 0 : 1;
 }
 
-// ---- block reductions (warp shuffles + one smem slot per warp) ----
-// red holds one slot per warp of the launch (blockDim.x / 32 <= 32).
-__device__ __forceinline__ int block_sum(int v, int* red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();  // red may still be read from the previous reduction
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    int s = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
-    return s;
-}
-
 // ---- thread groups: one CTA, or a thread-block cluster of CL CTAs cooperating on one
 // trajectory (global-storage mode).  Group-wide barriers are __syncthreads or the
 // cluster barrier (release/acquire at cluster scope, which orders the global-memory

@@ -11,7 +11,6 @@
 //                  AnalogSAT/cpu_sat/CpuSat.cpp:65-94,136-173,199-241).
 //  rhs_batch_kernel   standalone RHS over many trajectories whose state lives in
 //                  HBM (ISat::GetDerivatives, AnalogSAT/solver/IODE.h).
-//  viol_batch_kernel  exact unsat counts for many states (ISat::GetClauseViolationCount).
 #pragma once
 
 #include <climits>
@@ -842,30 +841,6 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
     for (; pr < npairs; pr += G) {
         const long long cnt = (2 * pr + 1 < ntraj ? 2 : 1) * stride;
         for (long long e = tid; e < cnt; e += BT) dxdt[(long long)(2 * pr) * stride + e] = nan;
-    }
-}
-
-// Exact unsat counts of many states: one CTA per state.
-template <typename T, int KMAX, bool EXACT, int BT, bool GS>
-__global__ void __launch_bounds__(BT) viol_batch_kernel(DevInstance I, const T* __restrict__ x,
-                                                         int* __restrict__ counts, int ntraj,
-                                                         long long stride, T* slab,
-                                                         long long slab_stride) {
-    constexpr int ENC = GS ? 1 : 0;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int red_i[32];
-    T* sy = GS ? slab + (long long)blockIdx.x * slab_stride : reinterpret_cast<T*>(smem_raw);
-    const int tid = threadIdx.x;
-    for (int tr = blockIdx.x; tr < ntraj; tr += gridDim.x) {
-        const T* X = x + (long long)tr * stride;
-        for (int i = tid; i < I.n; i += BT) sy[__ldg(I.iperm + i)] = X[i];
-        if (tid == 0) sy[I.n] = T(-1);
-        __syncthreads();
-        int cnt = 0;
-        for (int m = tid; m < I.m; m += BT) cnt += clause_violated<KMAX, EXACT, ENC>(I, m, sy);
-        cnt = block_sum(cnt, red_i);
-        if (tid == 0) counts[tr] = cnt;
-        __syncthreads();
     }
 }
 
