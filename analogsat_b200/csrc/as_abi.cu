@@ -22,6 +22,7 @@
 #include "as_fast.cuh"
 #include "as_kernels.cuh"
 #include "as_problem.h"
+#include "as_rows.cuh"
 #include "as_stream.cuh"
 #include "as_viol.cuh"
 
@@ -68,7 +69,7 @@ struct DevBuf {
 // Device copy of one or more packed instances in a single pool.
 struct DevicePool {
     int device = -1;
-    DevBuf lit, litw, slotw, srow, perm, iperm, icperm, cperm, inst, flit;
+    DevBuf lit, litw, slotw, srow, perm, iperm, icperm, cperm, deg, inst, flit;
     DevBuf plit, pc0, psrow, pcnt, picperm;  // clause-parts layouts (lean global-rows form)
     std::vector<DevInstance> host_inst;
 
@@ -96,6 +97,7 @@ struct DevicePool {
         AS_CUDA(srow.alloc(std::max<size_t>(nr, 1) * 4));
         AS_CUDA(perm.alloc(std::max<size_t>(np, 1) * 4));
         AS_CUDA(iperm.alloc(std::max<size_t>(np, 1) * 4));
+        AS_CUDA(deg.alloc(std::max<size_t>(np, 1) * 4));
         AS_CUDA(icperm.alloc(std::max<size_t>(nc, 1) * 4));
         AS_CUDA(cperm.alloc(std::max<size_t>(nc, 1) * 4));
         AS_CUDA(inst.alloc(sizeof(DevInstance) * std::max<size_t>(pk.size(), 1)));
@@ -171,6 +173,7 @@ struct DevicePool {
             d.srow = srow.as<int32_t>() + orr;
             d.perm = perm.as<int32_t>() + op;
             d.iperm = iperm.as<int32_t>() + op;
+            d.deg = deg.as<int32_t>() + op;
             d.icperm = icperm.as<int32_t>() + oc;
             d.cperm = cperm.as<int32_t>() + oc;
             {
@@ -193,7 +196,7 @@ struct DevicePool {
             int r;
             if ((r = put(lit, ol, q->lit)) || (r = put(litw, ow, q->litw)) || (r = put(slotw, ow, q->slotw)) ||
                 (r = put(srow, orr, q->srow)) || (r = put(perm, op, q->perm)) ||
-                (r = put(iperm, op, q->iperm)) || (r = put(icperm, oc, q->icperm)) ||
+                (r = put(iperm, op, q->iperm)) || (r = put(deg, op, q->deg)) || (r = put(icperm, oc, q->icperm)) ||
                 (r = put(cperm, oc, q->cperm)))
                 return r;
             ol += q->lit.size();
@@ -626,36 +629,6 @@ int ensure_uploaded(as_problem* p, int prec) {
     return p->dev[prec].upload(v, dev);
 }
 
-// Grid-stride launch of a per-state kernel: the shared-memory form when the state
-// fits one SM, else the global-storage form with a per-CTA slab owned by the problem
-// handle (grown on demand; calls on one handle must not overlap).
-template <typename T, typename OUT>
-int launch_per_state(as_problem* p, int prec, void (*fs)(DevInstance, const T*, OUT*, int, long long, T*, long long),
-                     void (*fg)(DevInstance, const T*, OUT*, int, long long, T*, long long), int bt,
-                     size_t vals, bool compact, const T* x, OUT* out, int ns, long long stride,
-                     cudaStream_t st) {
-    int dev = 0, sms = 0, optin = 0, occ = 0;
-    AS_CUDA(cudaGetDevice(&dev));
-    AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t smem = vals * sizeof(T);
-    if (compact && smem + 1024 <= (size_t)optin) {
-        AS_CUDA(raise_smem_limit((const void*)fs, smem));
-        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs, bt, smem));
-        const int grid = std::max(1, std::min(ns, sms * std::max(occ, 1)));
-        fs<<<grid, bt, smem, st>>>(p->dev[prec].host_inst[0], x, out, ns, stride, (T*)nullptr, 0ll);
-    } else {
-        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fg, bt, 0));
-        const int grid = std::max(1, std::min(ns, sms * std::max(occ, 1)));
-        const long long slab_stride = (long long)((vals + 63) / 64 * 64);
-        AS_CUDA(p->slab[prec].alloc((size_t)grid * slab_stride * sizeof(T)));
-        fg<<<grid, bt, 0, st>>>(p->dev[prec].host_inst[0], x, out, ns, stride, p->slab[prec].as<T>(),
-                                 slab_stride);
-    }
-    AS_CUDA(cudaGetLastError());
-    return AS_OK;
-}
-
 // Two states per CTA pass with packed FP32x2 arithmetic (FP32, compact instances whose
 // pair-kernel footprint fits one SM's shared memory); *done = false leaves the call to
 // the one-state kernel.
@@ -663,15 +636,16 @@ template <bool LOGA, int KMAX, bool EXACT>
 int launch_rhs_pair(as_problem* p, const float* x, float* d, int ns, cudaStream_t st, bool* done) {
     constexpr int BT = 1024;
     *done = false;
+    constexpr int CPT = 5, VPT = 1;  // instances whose footprint fits have M <= 5 * 1024
     if ((reinterpret_cast<uintptr_t>(x) & 3u) || !p->standard_model()) return AS_OK;
+    if (p->host.m > CPT * BT || p->host.n > VPT * BT) return AS_OK;
     const auto& q = p->packed(kLayoutPair);
     int dev = 0, sms = 0, optin = 0, occ = 0;
     AS_CUDA(cudaGetDevice(&dev));
     AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const size_t smem = rhs2_smem_bytes(q.n, q.m, q.nslots);
-    constexpr int CPT = 5, VPT = 1;  // instances whose footprint fits have M <= 5 * 1024
-    if (!q.compact || smem + 1024 > (size_t)optin || q.m > CPT * BT || q.n > VPT * BT) return AS_OK;
+    if (!q.compact || smem + 1024 > (size_t)optin) return AS_OK;
     int r = ensure_uploaded(p, kLayoutPair);
     if (r) return r;
     auto fn = &rhs_pair_kernel<LOGA, KMAX, EXACT, BT, CPT, VPT>;
@@ -693,6 +667,40 @@ int launch_rhs_pair(as_problem* p, const float* x, float* d, int ns, cudaStream_
     return AS_OK;
 }
 
+// States of an instance that fits no SM (as_rows.cuh): chunks of state groups, three
+// kernels per chunk.  The rows of a chunk's groups live in a slab owned by the problem
+// handle (grown on demand; calls on one handle must not overlap), about 64 MB -- half of
+// L2 -- or one group's where that is more.
+template <typename T, bool LOGA, int KMAX, bool EXACT, int SUB, int R>
+int launch_rhs_rows(as_problem* p, int prec, const T* x, T* d, int ns, cudaStream_t st) {
+    constexpr int L = SUB * R;
+    RowArgs<T> A;
+    A.I = p->dev[prec].host_inst[0];
+    A.x = x;
+    A.dxdt = d;
+    A.stride = (long long)A.I.n + A.I.m;
+    auto rounded = [](long long v) { return (v + 63) / 64 * 64; };  // groups start on a sector
+    A.sy_stride = rounded(((long long)A.I.n + 1) * L);
+    A.cs_stride = rounded(((long long)A.I.nslots + 1) * L);
+    const long long group_bytes = (A.sy_stride + A.cs_stride) * (long long)sizeof(T);
+    const int groups = (ns + L - 1) / L;
+    const int chunk = (int)std::max(1ll, std::min({(long long)groups, 65535ll, (64ll << 20) / group_bytes}));
+    AS_CUDA(p->slab[prec].alloc((size_t)chunk * group_bytes));
+    A.sy = p->slab[prec].template as<T>();
+    A.cs = A.sy + chunk * A.sy_stride;
+    for (int g = 0; g < groups; g += chunk) {
+        A.s0 = (long long)g * L;
+        A.ns = (int)std::min<long long>(ns - A.s0, (long long)chunk * L);
+        const int gy = (A.ns + L - 1) / L;
+        row_spread_kernel<T, L><<<dim3((A.I.n + 256) / 256, gy), 256, 0, st>>>(A);
+        row_clause_kernel<T, LOGA, KMAX, EXACT, SUB, R>
+            <<<dim3((unsigned)(((long long)R * A.I.m + 255) / 256), gy), 256, 0, st>>>(A);
+        row_var_kernel<T, SUB, R><<<dim3((unsigned)(((long long)R * A.I.n + 255) / 256), gy), 256, 0, st>>>(A);
+    }
+    AS_CUDA(cudaGetLastError());
+    return AS_OK;
+}
+
 template <typename T, bool LOGA, int KMAX, bool EXACT>
 int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
     constexpr int BT = 512;
@@ -703,10 +711,35 @@ int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
         if (r || done) return r;
     }
     const auto& q = p->packed(prec);
-    return launch_per_state<T, T>(p, prec, &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, false>,
-                                  &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, true>, BT,
-                                  rhs_smem_values(q.n, q.m, q.nslots), q.compact, x, d, ns,
-                                  (long long)(q.n + q.m), st);
+    int dev = 0, sms = 0, optin = 0, occ = 0;
+    AS_CUDA(cudaGetDevice(&dev));
+    AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const size_t vals = rhs_smem_values(q.n, q.m, q.nslots), smem = vals * sizeof(T);
+    const long long stride = (long long)q.n + q.m;
+    if (q.compact && smem + 1024 <= (size_t)optin) {  // one state per CTA pass, in shared memory
+        auto fs = &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, false>;
+        AS_CUDA(raise_smem_limit((const void*)fs, smem));
+        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs, BT, smem));
+        const int grid = std::max(1, std::min(ns, sms * std::max(occ, 1)));
+        fs<<<grid, BT, smem, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, (T*)nullptr, 0ll);
+    } else if (p->standard_model()) {
+        // Lanes per row: a 32-byte sector once there are states for most of it.
+        constexpr int V = 16 / (int)sizeof(T);  // lanes per 16-byte access
+        if (ns == 1) return launch_rhs_rows<T, LOGA, KMAX, EXACT, 1, 1>(p, prec, x, d, ns, st);
+        if (ns <= V) return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 1>(p, prec, x, d, ns, st);
+        return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 2>(p, prec, x, d, ns, st);
+    } else {  // tanh variant or bias term: one CTA per state, its vectors in a global slab
+        auto fg = &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, true>;
+        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fg, BT, 0));
+        const int grid = std::max(1, std::min(ns, sms * std::max(occ, 1)));
+        const long long slab_stride = (long long)((vals + 63) / 64 * 64);
+        AS_CUDA(p->slab[prec].alloc((size_t)grid * slab_stride * sizeof(T)));
+        fg<<<grid, BT, 0, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, p->slab[prec].template as<T>(),
+                                slab_stride);
+    }
+    AS_CUDA(cudaGetLastError());
+    return AS_OK;
 }
 
 template <typename T, bool LOGA>

@@ -34,6 +34,7 @@ struct DevInstance {
     const int32_t* iperm;   // public -> internal variable
     const int32_t* icperm;  // public -> internal clause
     const int32_t* cperm;   // internal -> public clause
+    const int32_t* deg;     // occurrences of an internal variable
     // CTDS variant (the reference's ISat implementations): tanh = 0 CpuSat / CudaSat,
     // tanh = 1 CpuSatTanh / CudaSatTanh with slope q; bias b (ISat::Set_B) adds
     // mean(a) (M/N) b knorm^2 (pi/2) sin(pi s_i) to ds_i (0: off).

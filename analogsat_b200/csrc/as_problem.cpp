@@ -836,7 +836,11 @@ PackedProblem pack(const HostProblem& p, int mode) {
         }
     }
     q.iperm.resize(p.n);
-    for (int v = 0; v < p.n; v++) q.iperm[q.perm[v]] = v;
+    q.deg.resize(p.n);
+    for (int v = 0; v < p.n; v++) {
+        q.iperm[q.perm[v]] = v;
+        q.deg[v] = degree[q.perm[v]];
+    }
 
     // SELL-32 rows: slice g is as wide as its largest degree
     q.srow.assign(q.nslices + 1, 0);

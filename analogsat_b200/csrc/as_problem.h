@@ -93,6 +93,7 @@ struct PackedProblem {
     std::vector<int32_t> iperm;    // public -> internal variable
     std::vector<int32_t> cperm;    // internal -> public clause
     std::vector<int32_t> icperm;   // public -> internal clause
+    std::vector<int32_t> deg;      // occurrences of an internal variable
     int max_degree = 0;
     long bank_wavefronts = 0;      // shared-memory wavefronts of one gather pass (>= 32-clause groups x k)
     // CTDS variant of the instance (ISat implementation and parameters): tanh = 1 is

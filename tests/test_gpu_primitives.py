@@ -45,3 +45,45 @@ def test_violation_counts_over_groups(n, m, lens, batch, dtype):
     got = A.clause_violation_counts(p, torch.from_numpy(x).cuda()).cpu().numpy()
     assert np.array_equal(got, counts(lits, length, x[:, :p.n]))
 
+
+def rhs(lits, lens, x, n, k, logspace):
+    """ds/dt and da/dt (or d log2 a / dt) of every state in 64 bits."""
+    x = x.astype(np.float64)
+    s, a = x[:, :n], np.exp2(x[:, n:]) if logspace else x[:, n:]
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]])
+    idx = np.repeat(np.arange(len(lens)), lens)
+    v, c = np.abs(lits) - 1, np.sign(lits).astype(np.float64)
+    f = 1 - c * s[:, v]
+    # the factors of missing literals are 1 - (-1) = 2
+    scale = 2.0 ** (k - lens) * 2.0 ** -k
+    K = np.multiply.reduceat(f, start, axis=1) * scale
+    out = np.zeros_like(x)
+    out[:, n:] = K * K / np.log(2) if logspace else a * K * K
+    for i in range(len(lits)):  # leave-one-out products
+        j = idx[i]
+        others = np.prod(np.delete(f[:, start[j]:start[j] + lens[j]], i - start[j], axis=1), axis=1) * scale[j]
+        out[:, v[i]] += 2 * a[:, j] * c[i] * others * K[:, j]
+    return out
+
+
+@pytest.mark.parametrize("dtype,logspace", [("float32", True), ("float32", False), ("float64", False)])
+@pytest.mark.parametrize("n,m,lens,batch", [
+    (33000, 250, [3], 1), (33000, 250, [4], 2), (40001, 333, [2, 3, 5], 3), (33000, 257, [3], 4),
+    (35000, 255, [3], 5), (33001, 400, [4], 8), (33000, 129, [1, 12], 9), (34000, 301, [3], 37)])
+def test_rhs_of_instances_beyond_one_sm(n, m, lens, batch, dtype, logspace):
+    lits, length = formula(n, m, lens, seed=n + m)
+    p = A.SatProblem.from_arrays(lits, length)
+    assert not p.layout_stats()["compact"]
+    rng = np.random.default_rng(2)
+    x = np.concatenate([rng.uniform(-1, 1, (batch, p.n)), rng.uniform(0.5, 3, (batch, p.m))], axis=1).astype(dtype)
+    got = A.get_derivatives(p, torch.from_numpy(x).cuda(), logspace=logspace).cpu().numpy()
+    want = rhs(lits, length, x, p.n, p.k, logspace)
+    # each contribution is a product of 2 k + 2 rounded factors (ex2.approx: 2 ulp more);
+    # a variable adds up at most its degree of them
+    deg = np.bincount(np.abs(lits) - 1).max()
+    eps = np.finfo(dtype).eps
+    big = np.abs(want).max(axis=1, keepdims=True)
+    assert (np.abs(got - want) <= (2 * max(lens) + deg + 8) * eps * big).all()
+    if dtype == "float64" and batch > 1:  # a state alone takes rows of one lane, the same operations
+        one = A.get_derivatives(p, torch.from_numpy(x[-1:]).cuda()).cpu().numpy()
+        assert np.array_equal(one[0], got[-1])
