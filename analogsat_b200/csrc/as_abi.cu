@@ -629,30 +629,36 @@ int ensure_uploaded(as_problem* p, int prec) {
     return p->dev[prec].upload(v, dev);
 }
 
-// Two states per CTA pass with packed FP32x2 arithmetic (FP32, compact instances whose
-// pair-kernel footprint fits one SM's shared memory); *done = false leaves the call to
-// the one-state kernel.
-template <bool LOGA, int KMAX, bool EXACT>
-int launch_rhs_pair(as_problem* p, const float* x, float* d, int ns, cudaStream_t st, bool* done) {
-    constexpr int BT = 1024;
+// The staged kernel (two FP32 states or one FP64 state per CTA pass; compact instances
+// whose footprint fits one SM's shared memory); *done = false leaves the call to the
+// other kernels.
+template <typename V, bool LOGA, int KMAX, bool EXACT, int BT>
+int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename Staged<V>::T* d, int ns,
+                      cudaStream_t st, bool* done) {
+    using T = typename Staged<V>::T;
+    constexpr int CPT = 5;  // instances whose footprint fits have M <= 5 * 1024
+    constexpr int layout = sizeof(T) == 8 ? AS_PREC_F64 : kLayoutPair;
     *done = false;
-    constexpr int CPT = 5, VPT = 1;  // instances whose footprint fits have M <= 5 * 1024
-    if ((reinterpret_cast<uintptr_t>(x) & 3u) || !p->standard_model()) return AS_OK;
-    if (p->host.m > CPT * BT || p->host.n > VPT * BT) return AS_OK;
-    const auto& q = p->packed(kLayoutPair);
+    if constexpr (BT < 1024)
+        if (p->host.n > BT || p->host.m > CPT * BT)
+            return launch_rhs_staged<V, LOGA, KMAX, EXACT, 2 * BT>(p, x, d, ns, st, done);
+    if ((reinterpret_cast<uintptr_t>(x) & (sizeof(T) - 1)) || !p->standard_model()) return AS_OK;
+    if (p->host.m > CPT * BT || p->host.n > BT) return AS_OK;
+    const auto& q = p->packed(layout);
     int dev = 0, sms = 0, optin = 0, occ = 0;
     AS_CUDA(cudaGetDevice(&dev));
     AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const size_t smem = rhs2_smem_bytes(q.n, q.m, q.nslots);
     if (!q.compact || smem + 1024 > (size_t)optin) return AS_OK;
-    int r = ensure_uploaded(p, kLayoutPair);
+    int r = ensure_uploaded(p, layout);
     if (r) return r;
-    auto fn = &rhs_pair_kernel<LOGA, KMAX, EXACT, BT, CPT, VPT>;
+    auto fn = &rhs_staged_kernel<V, LOGA, KMAX, EXACT, BT, CPT>;
     AS_CUDA(raise_smem_limit((const void*)fn, smem));
     AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, BT, smem));
     if (occ < 1) return AS_OK;
-    const int grid = std::max(1, std::min((ns + 1) / 2, sms * occ));
+    const int passes = (ns + Staged<V>::kRows - 1) / Staged<V>::kRows;
+    const int grid = std::max(1, std::min(passes, sms * occ));
     // bulk stores need dxdt congruent with x mod 16 bytes (same staging offsets)
     const int bulk_out = ((reinterpret_cast<uintptr_t>(x) - reinterpret_cast<uintptr_t>(d)) & 15u) == 0;
     if (p->rhs_status_dev != dev) {
@@ -660,8 +666,8 @@ int launch_rhs_pair(as_problem* p, const float* x, float* d, int ns, cudaStream_
         AS_CUDA(cudaMemset(p->rhs_status.p, 0, sizeof(int)));
         p->rhs_status_dev = dev;
     }
-    fn<<<grid, BT, smem, st>>>(p->dev[kLayoutPair].host_inst[0], x, d, ns, (long long)(q.n + q.m),
-                               bulk_out, p->rhs_status.as<int>());
+    fn<<<grid, BT, smem, st>>>(p->dev[layout].host_inst[0], x, d, ns, (long long)(q.n + q.m), bulk_out,
+                               p->rhs_status.as<int>());
     AS_CUDA(cudaGetLastError());
     *done = true;
     return AS_OK;
@@ -705,9 +711,10 @@ template <typename T, bool LOGA, int KMAX, bool EXACT>
 int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
     constexpr int BT = 512;
     constexpr int prec = sizeof(T) == 8 ? AS_PREC_F64 : AS_PREC_F32_LOGA;
-    if constexpr (sizeof(T) == 4 && EXACT) {
+    if constexpr (EXACT) {
+        using V = std::conditional_t<sizeof(T) == 8, double, float2>;
         bool done = false;
-        const int r = launch_rhs_pair<LOGA, KMAX, EXACT>(p, x, d, ns, st, &done);
+        const int r = launch_rhs_staged<V, LOGA, KMAX, EXACT, 128>(p, x, d, ns, st, &done);
         if (r || done) return r;
     }
     const auto& q = p->packed(prec);

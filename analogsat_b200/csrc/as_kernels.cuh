@@ -9,8 +9,8 @@
 //                  (AnalogSAT/solver/SatSolver.h:273-355,
 //                  AnalogSAT/cpu_sat/CpuRungeKutta.cpp:66-100,181-267,
 //                  AnalogSAT/cpu_sat/CpuSat.cpp:65-94,136-173,199-241).
-//  rhs_batch_kernel   standalone RHS over many trajectories whose state lives in
-//                  HBM (ISat::GetDerivatives, AnalogSAT/solver/IODE.h).
+//  rhs_staged_kernel, rhs_batch_kernel   standalone RHS over many trajectories whose state
+//                  lives in HBM (ISat::GetDerivatives, AnalogSAT/solver/IODE.h).
 #pragma once
 
 #include <climits>
@@ -520,26 +520,37 @@ __global__ void __launch_bounds__(BT) rhs_batch_kernel(DevInstance I, const T* _
 }
 
 // ---------------------------------------------------------------------------
-// Standalone batched RHS, two states per CTA pass (FP32): the spins and the clause
-// contributions are held as float2 pairs, so the literal loads, index arithmetic and
-// loop control are shared by the two states and the arithmetic runs as packed FP32x2
-// (FFMA2/FMUL2/FADD2).  Products are formed in the one-state kernel's order (2 r =
-// (km knorm)(2 a) is exact scaling).
+// Standalone batched RHS with staged states: one element type V of 8 bytes per shared
+// array element -- float2: two FP32 states per CTA pass, so the literal loads, index
+// arithmetic and loop control are shared by the two and the arithmetic runs as packed
+// FP32x2 (FFMA2/FMUL2/FADD2); double: one FP64 state.  Products are formed in the one-state
+// kernel's order.
 //
-// Data movement: two consecutive public states (contiguous in HBM) arrive in a shared
+// Data movement: the public states of a pass (contiguous in HBM) arrive in a shared
 // staging buffer with one 1-D bulk copy (cp.async.bulk, mbarrier completion) that is
-// issued one pair ahead by lane 0 of the last warp; the < 16-byte ragged ends of a row
-// pair that does not start on a 16-byte boundary are fetched with plain loads.  The kernel then works in the
+// issued one pass ahead by lane 0 of the last warp; the < 16-byte ragged ends of rows
+// that do not start on a 16-byte boundary are fetched with plain loads.  The kernel then works in the
 // public layout in place: a_m is read from and da_m written to its public position
 // (the pair packing makes the 32 clauses of a warp hit 32 different banks there), ds
-// is scattered to the public spin positions, and the finished pair leaves with one
+// is scattered to the public spin positions, and the finished rows leave with one
 // bulk store (when dxdt and x are congruent mod 16 bytes; plain coalesced stores
-// otherwise).  Two staging buffers alternate: pair i is stored from one while pair
-// i+1 lands in the other.  Two barriers per pair: one after the clause phase, one after
-// the variable phase, which also permutes the next pair's spins (its buffer has landed).  A wait that does not complete within two seconds (it
-// cannot, short of a broken device) turns every output of the CTA's remaining pairs
+// otherwise).  Two staging buffers alternate: pass i is stored from one while pass
+// i+1 lands in the other.  Two barriers per pass: one after the clause phase, one after
+// the variable phase, which also permutes the next pass's spins (its buffer has landed).  A wait that does not complete within two seconds (it
+// cannot, short of a broken device) turns every output of the CTA's remaining passes
 // into NaN and sets *status to 1 instead of hanging.
-// Shared layout: 2 mbarriers | staging[2] (2 stride + 3 floats each) | sy2 | cs2.
+// Shared layout: 2 mbarriers | staging[2] (2 stride + 3 floats each) | sy | cs.
+//
+// CTA size BT: the smallest of 128, 256, 512 and 1,024 with N <= BT and M <= 5 BT (a thread's
+// literal words stay in registers), so that small instances run several CTAs per SM, each
+// with its threads busy, instead of CTAs of 1,024 threads that mostly wait: 16,384 FP32
+// states of N = 50 / 120 / 200 / 400 (alpha 4.2) took 71 / 87 / 108 / 129 us with 1,024 threads,
+// 19 / 28 / 45 / 84 us so.
+// FP64, 1,999 states of N = 777, M = 3301: 104 us with the one-state kernel (no room for a
+// second CTA on the SM, so its loads, phases and stores run one after another), 63 us here =
+// 2.1 TB/s; 16,384 states of N = 120: 122 us against 68.  Bound by shared-memory wavefronts
+// (gathers, slot stores and sums: about 4,500 per FP32 pair of N = 1000, M = 4250) and, around
+// them, by two barriers a pass.
 // ---------------------------------------------------------------------------
 __host__ __device__ inline size_t rhs2_stage_floats(long long stride) {
     return (size_t)((2 * stride + 3 + 3) & ~3ll);
@@ -550,6 +561,70 @@ __host__ __device__ inline size_t rhs2_smem_bytes(int n, int m, int nslots) {
 }
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+
+// The states of a pass as one value per element.
+template <typename V> struct Staged;
+template <> struct Staged<float2> {
+    using T = float;
+    static constexpr int kRows = 2;
+    static __device__ __forceinline__ float2 splat(float a) { return f2(a); }
+    static __device__ __forceinline__ float2 get(const float* r0, const float* r1, int e) {
+        return make_float2(r0[e], r1[e]);
+    }
+    static __device__ __forceinline__ void put(float* r0, float* r1, int e, float2 v) {
+        r0[e] = v.x;
+        r1[e] = v.y;
+    }
+    static __device__ __forceinline__ float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+    static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+    // c = -c_lit = +1 for a negated literal, -1 otherwise (from the sign bit):
+    // f = 1 - c_lit s = 1 + c s
+    static __device__ __forceinline__ float2 factor(uint32_t w, float2 s) {
+        return __ffma2_rn(f2(__int_as_float((w & 0x80000000u) ^ 0xBF800000u)), s, f2(1.0f));
+    }
+    // The power-of-two scalings (kn = 2^-k) folded, the same roundings above the subnormals:
+    // with P = f_0 .. f_{k-1}, K_m = kn P and -2 r = -2 (K_m kn) a_m = P (a_m (-2 kn^2)); the
+    // contribution c_lit 2 r K_mi is then (-2 r K_mi) c.
+    static __device__ __forceinline__ float2 product(float2 km, float2 f, bool first) {
+        return first ? f : __fmul2_rn(km, f);
+    }
+    static __device__ __forceinline__ float2 weight(float2 P, float kn, float2 am) {
+        return __fmul2_rn(P, __fmul2_rn(am, f2(-2.0f * kn * kn)));
+    }
+    static __device__ __forceinline__ float2 dlog(float2 P, float kn) {  // K_m^2 / ln 2
+        return __fmul2_rn(__fmul2_rn(P, P), f2(kn * kn * kInvLn2));
+    }
+    static __device__ __forceinline__ float2 da(float2 P, float kn, float2 am) {  // (a_m K_m) K_m
+        return __fmul2_rn(__fmul2_rn(__fmul2_rn(am, f2(kn * kn)), P), P);
+    }
+    static __device__ __forceinline__ float2 contribution(float2 r, float2 prod, uint32_t w) {
+        return __fmul2_rn(__fmul2_rn(r, prod), f2(__int_as_float((w & 0x80000000u) ^ 0xBF800000u)));
+    }
+};
+template <> struct Staged<double> {
+    using T = double;
+    static constexpr int kRows = 1;
+    static __device__ __forceinline__ double splat(double a) { return a; }
+    static __device__ __forceinline__ double get(const double* r0, const double*, int e) { return r0[e]; }
+    static __device__ __forceinline__ void put(double* r0, double*, int e, double v) { r0[e] = v; }
+    static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ double flip(double a, uint32_t w) {  // -a for a negated literal
+        return __hiloint2double(__double2hiint(a) ^ (int)(w & 0x80000000u), __double2loint(a));
+    }
+    static __device__ __forceinline__ double factor(uint32_t w, double s) { return __dsub_rn(1.0, flip(s, w)); }
+    static __device__ __forceinline__ double product(double km, double f, bool) { return __dmul_rn(km, f); }
+    static __device__ __forceinline__ double weight(double km, double kn, double am) {
+        return __dmul_rn(__dmul_rn(km, kn), am);
+    }
+    static __device__ __forceinline__ double da(double km, double, double am) {
+        return __dmul_rn(__dmul_rn(am, km), km);
+    }
+    static __device__ __forceinline__ double contribution(double r, double prod, uint32_t w) {
+        const double rr = __dmul_rn(r, prod);
+        return flip(__dadd_rn(rr, rr), w);
+    }
+};
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -602,52 +677,59 @@ __device__ __forceinline__ void bulk_wait_read() {
 }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// Row pair `pr` of x as it lands in the staging buffer: stg[off + e] = x[2 pr stride + e].
-struct PairCopy {
-    const float* src;
-    int cnt;   // floats (one or two rows)
+// Rows `pr` (the states of a pass) of x as they land in the staging buffer:
+// stg[off + e] = x[kRows pr stride + e].
+template <typename T, int ROWS>
+struct PassCopy {
+    static constexpr int kVec = 16 / (int)sizeof(T);
+    const T* src;
+    int cnt;   // values (one or two rows)
     int off;   // staging offset, keeps shared and global addresses congruent mod 16
-    int head;  // plain-loaded floats before the first 16-byte boundary
-    int nb;    // floats moved by the bulk copy (multiple of 4)
-    __device__ PairCopy(const float* x, int pr, int ntraj, long long stride) {
-        src = x + (long long)(2 * pr) * stride;
-        cnt = (int)((2 * pr + 1 < ntraj ? 2 : 1) * stride);
+    int head;  // plain-loaded values before the first 16-byte boundary
+    int nb;    // values moved by the bulk copy (16-byte units)
+    __device__ PassCopy(const T* x, int pr, int ntraj, long long stride) {
+        src = x + (long long)(ROWS * pr) * stride;
+        cnt = (int)((ROWS == 2 && 2 * pr + 1 < ntraj ? 2 : 1) * stride);
         const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u);
-        off = (int)(mis >> 2);
-        head = min(cnt, (int)(((16u - mis) & 15u) >> 2));
-        nb = ((cnt - head) >> 2) << 2;
+        off = (int)(mis / sizeof(T));
+        head = min(cnt, (int)(((16u - mis) & 15u) / sizeof(T)));
+        nb = (cnt - head) / kVec * kVec;
     }
-    // thread t < 6 owns one ragged float: t < 3 in the head, 3..5 in the tail
+    // thread t < kRagged owns one ragged value: the first half in the head, the rest in the tail
+    static constexpr int kRagged = 2 * (kVec - 1);
     __device__ int ragged(int t) const {
-        const int e = t < 3 ? t : head + nb + (t - 3);
-        return (t < 3 ? e < head : e < cnt) ? e : -1;
+        const int e = t < kVec - 1 ? t : head + nb + (t - (kVec - 1));
+        return (t < kVec - 1 ? e < head : e < cnt) ? e : -1;
     }
 };
 
-// CPT / VPT: clauses / variables per thread (M <= CPT * BT, N <= VPT * BT); a thread's
-// literal words, public clause and variable indices and SELL rows are the same for
-// every pair, so they are loaded once into registers.
-template <bool LOGA, int KMAX, bool EXACT, int BT, int CPT, int VPT>
-__global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const float* __restrict__ x,
-                                                          float* __restrict__ dxdt, int ntraj,
-                                                          long long stride, int bulk_out,
-                                                          int* __restrict__ status) {
+// CPT: clauses per thread (M <= CPT BT, N <= BT); a thread's literal words, public clause
+// and variable indices and SELL rows are the same for every pass, so they are loaded once
+// into registers.
+template <typename V, bool LOGA, int KMAX, bool EXACT, int BT, int CPT>
+__global__ void __launch_bounds__(BT, 1024 / BT)
+    rhs_staged_kernel(DevInstance I, const typename Staged<V>::T* __restrict__ x,
+                      typename Staged<V>::T* __restrict__ dxdt, int ntraj, long long stride, int bulk_out,
+                      int* __restrict__ status) {
+    using O = Staged<V>;
+    using T = typename O::T;
+    constexpr int ROWS = O::kRows;
+    using Copy = PassCopy<T, ROWS>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
-    const size_t sf = rhs2_stage_floats(stride);
-    float* stg0 = reinterpret_cast<float*>(smem_raw + 16);
-    float2* sy = reinterpret_cast<float2*>(stg0 + 2 * sf);
-    float2* cs = sy + ((I.n + 1 + 3) & ~3);
+    const size_t sf = rhs2_stage_floats(stride) * 4 / sizeof(T);
+    T* stg0 = reinterpret_cast<T*>(smem_raw + 16);
+    V* sy = reinterpret_cast<V*>(stg0 + 2 * sf);
+    V* cs = sy + ((I.n + 1 + 3) & ~3);
     const int tid = threadIdx.x;
     const int n = I.n;
-    const float knorm = (float)ldexp(1.0, -I.k);
-    const float2 kn2 = f2(knorm);
-    const int npairs = (ntraj + 1) / 2;
+    const T knorm = (T)ldexp(1.0, -I.k);
+    const int npairs = (ntraj + ROWS - 1) / ROWS;  // passes
     const int G = gridDim.x;
     constexpr unsigned long long kWaitNs = 2000000000ull;
     int pr = blockIdx.x;
     if (pr >= npairs) return;
-    for (int j = tid; j <= I.nslots; j += BT) cs[j] = f2(0.0f);
+    for (int j = tid; j <= I.nslots; j += BT) cs[j] = O::splat(T(0));
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_init(bar + 1, 1);
@@ -663,45 +745,38 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
             if (m < I.m && (EXACT || q < I.k)) lw[i][q].load(I, q * I.mp + m);
             else lw[i][q].w = 0;
     }
-    int vp[VPT];
-    uint32_t vrows[VPT];  // first row | end row << 16 (rows < 2048 for compact instances)
-#pragma unroll
-    for (int i = 0; i < VPT; i++) {
-        const int v = tid + i * BT;
-        vp[i] = v < n ? __ldg(I.perm + v) : 0;
-        vrows[i] = v < n ? (uint32_t)ld_ro(I.srow + (v >> 5)) | ((uint32_t)ld_ro(I.srow + (v >> 5) + 1) << 16) : 0u;
-    }
-    if (tid == 0) sy[n] = f2(-1.0f);
+    const bool has_v = tid < n;  // one variable per thread
+    const int vp = has_v ? __ldg(I.perm + tid) : 0;
+    const int r0 = has_v ? ld_ro(I.srow + (tid >> 5)) : 0, r1 = has_v ? ld_ro(I.srow + (tid >> 5) + 1) : 0;
+    if (tid == 0) sy[n] = O::splat(T(-1));
     __syncthreads();
     // All bulk copies and stores are issued by lane 0 of the last warp (IO), so that the
     // store -> reuse wait falls on a warp with no more clauses than the first.  Copy of
-    // pair q into buffer b: IO starts the bulk part; after it, lanes 0..5 of the same
+    // pass q into buffer b: IO starts the bulk part; after it, the first lanes of the same
     // warp load the < 16-byte ragged ends and store them into the buffer (positions the
-    // bulk copy does not write).  The buffer's previous pair has left it by then: IO
+    // bulk copy does not write).  The buffer's previous pass has left it by then: IO
     // waited for its bulk store to read out, and __syncwarp orders the lanes after it.
     constexpr int IO = BT - 32;
     const bool io_warp = tid >= IO;
     auto issue = [&](int q, int b) {
-        const PairCopy c(x, q, ntraj, stride);
-        float* dst = stg0 + (size_t)b * sf;
+        const Copy c(x, q, ntraj, stride);
+        T* dst = stg0 + (size_t)b * sf;
         if (tid == IO) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive_tx(bar + b, (uint32_t)c.nb * 4u);
-            if (c.nb > 0) bulk_load(dst + c.off + c.head, c.src + c.head, (uint32_t)c.nb * 4u, bar + b);
+            mbar_arrive_tx(bar + b, (uint32_t)c.nb * (uint32_t)sizeof(T));
+            if (c.nb > 0) bulk_load(dst + c.off + c.head, c.src + c.head, (uint32_t)c.nb * (uint32_t)sizeof(T), bar + b);
         }
-        if ((unsigned)(tid - IO) < 6u) {  // lanes 0..5 of the IO warp
+        if ((unsigned)(tid - IO) < (unsigned)Copy::kRagged) {
             const int e = c.ragged(tid - IO);
             if (e >= 0) dst[c.off + e] = __ldg(c.src + e);
         }
     };
-    // Spins of the pair in buffer b into internal order, interleaved.
+    // Spins of the pass in buffer b into internal order, interleaved.
     auto permute = [&](int q, int b) {
-        const PairCopy c(x, q, ntraj, stride);
-        const float* A0 = stg0 + (size_t)b * sf + c.off;
-        const float* A1 = 2 * q + 1 < ntraj ? A0 + stride : A0;
-#pragma unroll
-        for (int i = 0; i < VPT; i++)
-            if (tid + i * BT < n) sy[tid + i * BT] = make_float2(A0[vp[i]], A1[vp[i]]);
+        const Copy c(x, q, ntraj, stride);
+        const T* A0 = stg0 + (size_t)b * sf + c.off;
+        const T* A1 = ROWS == 2 && 2 * q + 1 < ntraj ? A0 + stride : A0;
+        if (has_v) sy[tid] = O::get(A0, A1, vp);
     };
     uint32_t parity = 0;   // bit b: phase parity expected next on bar[b]
     uint32_t pending = 1;  // bit b: a copy into buffer b not yet waited for (same in all threads)
@@ -716,58 +791,48 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
     __syncthreads();  // the ragged ends stored by the IO warp
     permute(pr, 0);
     bool failed = __syncthreads_or(!ok);
-    // Per pair: clause phase | barrier | next pair's copy waited for | variable phase of
-    // this pair and spin permutation of the next (independent work in one phase) |
-    // barrier + timeout vote | this pair stored, the pair after next copied in.
+    // Per pass: clause phase | barrier | next pass's copy waited for | variable phase of
+    // this pass and spin permutation of the next (independent work in one phase) |
+    // barrier + timeout vote | this pass stored, the pass after next copied in.
     for (int it = 0; !failed && pr < npairs; pr += G, it++) {
         const int b = it & 1;
-        const bool two = 2 * pr + 1 < ntraj;
-        const PairCopy cur(x, pr, ntraj, stride);
-        float* S0 = stg0 + (size_t)b * sf + cur.off;
-        float* S1 = two ? S0 + stride : S0;
+        const bool two = ROWS == 2 && 2 * pr + 1 < ntraj;
+        const Copy cur(x, pr, ntraj, stride);
+        T* S0 = stg0 + (size_t)b * sf + cur.off;
+        T* S1 = two ? S0 + stride : S0;
         // clause phase: a_m in, da_m out at the public clause position
 #pragma unroll
         for (int i = 0; i < CPT; i++) {
             if (tid + i * BT >= I.m) break;
             const Lit<0>* w = lw[i];
-            float2 f[KMAX];
-            float2 km = kn2;
+            V f[KMAX];
+            V km = O::splat(knorm);
             const int j = lj[i];
 #pragma unroll
             for (int q = 0; q < KMAX; q++) {
                 if (EXACT || q < I.k) {
-                    // c = -c_lit = +1 for a negated literal, -1 otherwise (from the sign bit):
-                    // f = 1 - c_lit s = 1 + c s
-                    const float c = __int_as_float((w[q].w & 0x80000000u) ^ 0xBF800000u);
-                    f[q] = __ffma2_rn(f2(c), sy[w[q].var()], f2(1.0f));
-                    km = __fmul2_rn(km, f[q]);
+                    f[q] = O::factor(w[q].w, sy[w[q].var()]);
+                    km = O::product(km, f[q], q == 0);
                 }
             }
-            const float2 a = make_float2(S0[j], S1[j]);
-            float2 am;
-            if constexpr (LOGA) am = make_float2(exp2_fast(a.x), exp2_fast(a.y));
-            else am = a;
-            // da: (km km) / ln 2 in log space, (a km) km otherwise, as in the one-state kernel
-            const float2 da = LOGA ? __fmul2_rn(__fmul2_rn(km, km), f2(kInvLn2))
-                                   : __fmul2_rn(__fmul2_rn(am, km), km);
-            S0[j] = da.x;
-            S1[j] = da.y;
-            // -2 r (exact scaling): the contribution c_lit 2 r K_mi is then (-2 r K_mi) c
-            const float2 r2n = __fmul2_rn(__fmul2_rn(km, kn2), __fmul2_rn(am, f2(-2.0f)));
+            V am = O::get(S0, S1, j);
+            if constexpr (LOGA) am = make_float2(exp2_fast(am.x), exp2_fast(am.y));
+            if constexpr (LOGA) O::put(S0, S1, j, O::dlog(km, knorm));
+            else O::put(S0, S1, j, O::da(km, knorm, am));
+            const V r = O::weight(km, knorm, am);
 #pragma unroll
             for (int q = 0; q < KMAX; q++) {
                 if (EXACT || q < I.k) {
-                    float2 prod = f2(1.0f);
+                    V prod = O::splat(T(1));
                     bool first = true;
 #pragma unroll
                     for (int l = 0; l < KMAX; l++) {
                         if (l != q && (EXACT || l < I.k)) {
-                            prod = first ? f[l] : __fmul2_rn(prod, f[l]);
+                            prod = first ? f[l] : O::mul(prod, f[l]);
                             first = false;
                         }
                     }
-                    const float c = __int_as_float((w[q].w & 0x80000000u) ^ 0xBF800000u);
-                    cs[w[q].slot()] = __fmul2_rn(__fmul2_rn(r2n, prod), f2(c));
+                    cs[w[q].slot()] = O::contribution(r, prod, w[q].w);
                 }
             }
         }
@@ -780,19 +845,14 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
             pending &= ~(1u << (b ^ 1));
         }
         // var phase: ds_i to the public spin position
-#pragma unroll
-        for (int i = 0; i < VPT; i++) {
-            const int v = tid + i * BT;
-            if (v >= n) break;
-            const int r0 = (int)(vrows[i] & 0xffffu), r1 = (int)(vrows[i] >> 16);
-            const float2* p = cs + r0 * 32 + (v & 31);
-            float2 sum = f2(0.0f);
+        if (has_v) {
+            const V* p = cs + r0 * 32 + (tid & 31);
+            V sum = O::splat(T(0));
 #pragma unroll 8
-            for (int r = r0; r < r1; r++, p += 32) sum = __fadd2_rn(sum, *p);
-            S0[vp[i]] = sum.x;
-            S1[vp[i]] = sum.y;
+            for (int r = r0; r < r1; r++, p += 32) sum = O::add(sum, *p);
+            O::put(S0, S1, vp, sum);
         }
-        // the next pair's spins (its buffer is the other one; sy is free: this pair's
+        // the next pass's spins (its buffer is the other one; sy is free: this pass's
         // clause phase has read it)
         if (more) permute(pr + G, b ^ 1);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // results -> bulk store
@@ -800,10 +860,10 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
             failed = true;
             break;
         }
-        float* D = dxdt + (long long)(2 * pr) * stride;
+        T* D = dxdt + (long long)(ROWS * pr) * stride;
         if (bulk_out) {
-            if (tid == IO && cur.nb > 0) bulk_store(D + cur.head, S0 + cur.head, (uint32_t)cur.nb * 4u);
-            if ((unsigned)(tid - IO) < 6u) {
+            if (tid == IO && cur.nb > 0) bulk_store(D + cur.head, S0 + cur.head, (uint32_t)cur.nb * (uint32_t)sizeof(T));
+            if ((unsigned)(tid - IO) < (unsigned)Copy::kRagged) {
                 const int e = cur.ragged(tid - IO);
                 if (e >= 0) D[e] = S0[e];
             }
@@ -812,7 +872,7 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
             __syncthreads();  // the buffer is read out before the copy into it
         }
         if (pr + 2 * G < npairs) {
-            // this buffer takes the pair after next once its store has read it out
+            // this buffer takes the pass after next once its store has read it out
             if (io_warp) {
                 if (tid == IO && bulk_out) bulk_wait_read();
                 __syncwarp();
@@ -837,10 +897,10 @@ __global__ void __launch_bounds__(BT, 1) rhs_pair_kernel(DevInstance I, const fl
         bulk_wait_all();
         atomicExch(status, 1);
     }
-    const float nan = __int_as_float(0x7fc00000);
+    const T nan = (T)__int_as_float(0x7fc00000);
     for (; pr < npairs; pr += G) {
-        const long long cnt = (2 * pr + 1 < ntraj ? 2 : 1) * stride;
-        for (long long e = tid; e < cnt; e += BT) dxdt[(long long)(2 * pr) * stride + e] = nan;
+        const long long cnt = (ROWS == 2 && 2 * pr + 1 < ntraj ? 2 : 1) * stride;
+        for (long long e = tid; e < cnt; e += BT) dxdt[(long long)(ROWS * pr) * stride + e] = nan;
     }
 }
 

@@ -647,7 +647,7 @@ def rhs_kernel_bench(A, problem, ics_dev, nm, st, reps=10):
     bytes_per_launch = B * 8 * nm + 4 * W["k"] * W["m"]
     # traffic: ncu dram__bytes_read + dram__bytes_write of one launch of this exact
     # configuration (profiles/rhs_pair_kernel_16384_states_N1000_M4250.md)
-    kernel = "rhs_pair_kernel" if x.dtype == torch.float32 else "rhs_batch_kernel"
+    kernel = "rhs_staged_kernel"
     return {"bound": "hbm", "kernel": kernel, "states_per_launch": B,
             "ms_per_launch": ms, "achieved": bytes_per_launch / (ms / 1e3) / 1e9, "unit": "GB/s",
             "bytes_per_launch": bytes_per_launch,

@@ -87,3 +87,32 @@ def test_rhs_of_instances_beyond_one_sm(n, m, lens, batch, dtype, logspace):
     if dtype == "float64" and batch > 1:  # a state alone takes rows of one lane, the same operations
         one = A.get_derivatives(p, torch.from_numpy(x[-1:]).cuda()).cpu().numpy()
         assert np.array_equal(one[0], got[-1])
+
+
+@pytest.mark.parametrize("dtype,logspace", [("float32", True), ("float32", False), ("float64", False)])
+@pytest.mark.parametrize("n,m,k,batch,shift", [
+    (3, 1, 3, 1, 0), (50, 210, 3, 301, 1), (256, 1280, 3, 7, 0), (257, 1280, 3, 7, 1), (200, 1281, 3, 8, 0),
+    (255, 700, 4, 2, 1), (512, 2560, 3, 301, 0), (513, 2160, 3, 5, 1), (400, 2561, 4, 3, 0), (999, 4251, 3, 298, 1),
+    (1024, 4100, 3, 4, 0)])
+def test_rhs_of_staged_states(n, m, k, batch, shift, dtype, logspace):
+    lits, lens, _ = make_instance("fast", n, m, k, seed=n + m)
+    p = A.SatProblem.from_arrays(lits, lens)
+    rng = np.random.default_rng(3)
+    x = np.concatenate([rng.uniform(-1, 1, (batch, p.n)), rng.uniform(0.5, 3, (batch, p.m))], axis=1).astype(dtype)
+    # rows off a 16-byte boundary, and an output that shares or does not share its offset
+    buf = torch.zeros(2, x.size + 4, dtype=getattr(torch, dtype), device="cuda")
+    xs = buf[0, shift:shift + x.size].view(x.shape)
+    xs.copy_(torch.from_numpy(x))
+    out = buf[1, 1:1 + x.size].view(x.shape)
+    A.get_derivatives(p, xs, out=out, logspace=logspace)
+    A.rhs_check(p)
+    got = out.cpu().numpy()
+    rows = [0, batch // 2, batch - 1]
+    want = rhs(lits, lens, x[rows], p.n, p.k, logspace)
+    deg = np.bincount(np.abs(lits) - 1).max()
+    big = np.abs(want).max(axis=1, keepdims=True)
+    assert (np.abs(got[rows] - want) <= (2 * k + deg + 8) * np.finfo(dtype).eps * big).all()
+    assert float(buf[1, 0]) == 0 and not buf[1, 1 + x.size:].any()  # nothing written around the output
+    for r in rows:  # a state alone: the same operations
+        one = A.get_derivatives(p, xs[r:r + 1].clone(), logspace=logspace).cpu().numpy()
+        assert np.array_equal(one[0], got[r])
