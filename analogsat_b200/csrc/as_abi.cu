@@ -19,6 +19,7 @@
 
 #include "../../include/analogsat_b200.h"
 #include "as_ingest.h"
+#include "as_adjoint.cuh"
 #include "as_fast.cuh"
 #include "as_kernels.cuh"
 #include "as_problem.h"
@@ -53,7 +54,12 @@ int fail(int code, const std::string& msg) {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    ~DevBuf() { if (p) cudaFree(p); }
+    ~DevBuf() { release(); }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        bytes = 0;
+    }
     cudaError_t alloc(size_t b) {
         if (b <= bytes && p) return cudaSuccess;
         if (p) cudaFree(p);
@@ -391,6 +397,19 @@ struct StreamPlan {
     ~StreamPlan() { if (graph) cudaGraphExecDestroy(graph); }
 };
 
+// Device buffers of as_solver_adjoint, kept between calls on one solver (grown on demand;
+// the checkpoint pool and the step tables are given back after a call that needed more
+// than kAdjointKeep bytes of them).
+constexpr size_t kAdjointKeep = 1ull << 30;
+struct AdjointPlan {
+    DevBuf ui, us, uw, w, hs, off, ns, used, loss, gx, gw, ck, hsc;
+    std::vector<int> traj;  // the trajectories that ui, us and uw describe
+    void trim() {
+        for (DevBuf* b : {&ck, &hs, &off})
+            if (b->bytes > kAdjointKeep) b->release();
+    }
+};
+
 struct as_solver {
     int device = 0;
     int precision = AS_PREC_F32_LOGA;
@@ -414,6 +433,7 @@ struct as_solver {
     int kernel_choice = AS_KERNEL_AUTO;  // AS_KERNEL_GENERIC: never the lean FP32 kernel
     int storage_mode = 0;  // 0 automatic, 1 shared memory, 2 global storage, 3 stream
     std::unique_ptr<StreamPlan> sp;  // streamed solver state
+    std::unique_ptr<AdjointPlan> ap; // adjoint buffers
     int stream_parts = 0;            // clause parts per stream pass (0 = from the L2 budget)
 
     // trajectories
@@ -2023,8 +2043,6 @@ int32_t as_solver_solve_noalloc(as_solver* s, int32_t problem_index, int32_t num
 // ---------------------------------------------------------------------------
 // Adjoint (gradients of the final potential)
 // ---------------------------------------------------------------------------
-#include "as_adjoint.cuh"
-
 namespace {
 
 using AdjFn = void (*)(AdjointParams);
@@ -2041,10 +2059,26 @@ struct AdjVariant {
 
 const std::vector<AdjVariant>& adj_variants() {
     static const std::vector<AdjVariant> v = {
-        AS_ADJ(float, AS_PREC_F32_LOGA, 3, true),  AS_ADJ(float, AS_PREC_F32_LOGA, 16, false),
-        AS_ADJ(double, AS_PREC_F64, 3, true),      AS_ADJ(double, AS_PREC_F64, 16, false),
+        AS_ADJ(float, AS_PREC_F32_LOGA, 3, true),  AS_ADJ(float, AS_PREC_F32_LOGA, 4, true),
+        AS_ADJ(float, AS_PREC_F32_LOGA, 16, false), AS_ADJ(double, AS_PREC_F64, 3, true),
+        AS_ADJ(double, AS_PREC_F64, 4, true),       AS_ADJ(double, AS_PREC_F64, 16, false),
     };
     return v;
+}
+
+// CTA size of an adjoint kernel.  The CTAs that share an SM -- as many as its shared memory
+// holds, but no more than give the same number of waves of units -- take its 1,024
+// threads at 64 registers together, each with the fewest threads that keep its clause
+// rounds (the last round nearly full).  1,024 units of N = 200, M = 850, FP32: forward,
+// four CTAs of 224 threads 0.98 ms (five of 192, also two waves, 1.26; one of 864 1.63);
+// backward, three of 288 2.24 ms (one of 864 2.91, 128-thread CTAs 3.47).
+int adjoint_threads(size_t smem, int m, int units, int sms, int smem_per_sm) {
+    const int fit = std::max(1, std::min(16, (int)((size_t)smem_per_sm / (smem + 2048))));
+    const int waves = (units + sms * fit - 1) / (sms * fit);
+    const int ctas = (units + sms * waves - 1) / (sms * waves);
+    const int target = 1024 / ctas / 32 * 32;
+    const int rounds = std::max(1, (m + target - 1) / target);
+    return std::max(64, std::min(1024, ((m + rounds - 1) / rounds + 31) / 32 * 32));
 }
 
 }  // namespace
@@ -2061,13 +2095,15 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     const int nt = s->num_traj;
     // one launch shape for all trajectories: the largest instance decides
     const AdjVariant* av = nullptr;
-    size_t vals = 0;
-    int bt = 64;
+    size_t limit = 0, fvals = 0, bvals = 0;
+    int mmax = 1;
     for (int t = 0; t < nt; t++) {
         const auto& q = s->problems[s->traj_problem[t]];
         if (!q.compact) return fail(AS_ERR_UNSUPPORTED, "adjoint: instance beyond the compact encoding");
-        vals = std::max(vals, adjoint_smem_values(q.n, q.m, q.nslots));
-        bt = std::max(bt, preferred_bt(q));
+        limit = std::max(limit, adjoint_limit_values(q.n, q.m, q.nslots));
+        fvals = std::max(fvals, adjoint_smem_values(q.n, q.m, q.nslots, false, weights != nullptr));
+        bvals = std::max(bvals, adjoint_smem_values(q.n, q.m, q.nslots, true, weights != nullptr));
+        mmax = std::max(mmax, q.m);
     }
     for (const auto& v : adj_variants()) {
         bool ok = v.precision == s->precision;
@@ -2078,98 +2114,123 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
         if (ok) { av = &v; break; }
     }
     if (!av) return fail(AS_ERR_UNSUPPORTED, "adjoint: clause length > 16");
-    const size_t smem = vals * av->bytes;
-    if (smem > s->smem_limit) return fail(AS_ERR_UNSUPPORTED, "adjoint: instance too large for one SM");
-
-    std::vector<int> ui(nt);
-    std::vector<long long> us(nt), uw(nt);
-    long long wtot = 0;
-    for (int t = 0; t < nt; t++) {
-        ui[t] = s->traj_problem[t];
-        us[t] = s->traj_off[t];
-        uw[t] = wtot;
-        wtot += s->problems[s->traj_problem[t]].m;
-    }
-    DevBuf d_ui, d_us, d_uw, d_w, d_hs, d_ns, d_loss, d_gx, d_gw, d_uc, d_ck;
     const size_t vb = av->bytes;
-    AS_CUDA(d_ui.alloc(sizeof(int) * nt));
-    AS_CUDA(d_us.alloc(sizeof(long long) * nt));
-    AS_CUDA(d_uw.alloc(sizeof(long long) * nt));
-    AS_CUDA(d_hs.alloc(sizeof(double) * (size_t)nt * max_steps));
-    AS_CUDA(d_ns.alloc(sizeof(int) * (nt + 2)));
-    AS_CUDA(d_loss.alloc(sizeof(double) * nt));
-    AS_CUDA(d_gx.alloc(vb * (size_t)s->total_values));
-    AS_CUDA(d_gw.alloc(sizeof(double) * (size_t)std::max<long long>(wtot, 1)));
-    AS_CUDA(cudaMemcpy(d_ui.p, ui.data(), sizeof(int) * nt, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(d_us.p, us.data(), sizeof(long long) * nt, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(d_uw.p, uw.data(), sizeof(long long) * nt, cudaMemcpyHostToDevice));
-    if (weights) {
-        AS_CUDA(d_w.alloc(sizeof(double) * (size_t)std::max<long long>(wtot, 1)));
-        AS_CUDA(cudaMemcpy(d_w.p, weights, sizeof(double) * wtot, cudaMemcpyHostToDevice));
+    if (limit * vb > s->smem_limit) return fail(AS_ERR_UNSUPPORTED, "adjoint: instance too large for one SM");
+
+    long long wtot = 0, etot = 0;
+    std::vector<long long> uw(nt);
+    for (int t = 0; t < nt; t++) {
+        const auto& q = s->problems[s->traj_problem[t]];
+        uw[t] = wtot;
+        wtot += q.m;
+        etot += q.n + q.m;
     }
-    AS_CUDA(cudaMemset(d_ns.p, 0, sizeof(int) * (nt + 2)));
+    if (!s->ap) s->ap.reset(new AdjointPlan());
+    AdjointPlan& A = *s->ap;
+    cudaStream_t st = s->stream;
+    AS_CUDA(A.hs.alloc(sizeof(double) * (size_t)nt * max_steps));
+    AS_CUDA(A.off.alloc(sizeof(long long) * (size_t)nt * (max_steps + 1)));
+    AS_CUDA(A.ns.alloc(sizeof(int) * (nt + 2)));
+    AS_CUDA(A.used.alloc(sizeof(unsigned long long)));
+    AS_CUDA(A.loss.alloc(sizeof(double) * nt));
+    AS_CUDA(A.gx.alloc(vb * (size_t)s->total_values));
+    AS_CUDA(A.gw.alloc(sizeof(double) * (size_t)std::max<long long>(wtot, 1)));
+    if (A.traj != s->traj_problem) {
+        A.traj.clear();
+        AS_CUDA(A.ui.alloc(sizeof(int) * nt));
+        AS_CUDA(A.us.alloc(sizeof(long long) * nt));
+        AS_CUDA(A.uw.alloc(sizeof(long long) * nt));
+        AS_CUDA(cudaMemcpyAsync(A.ui.p, s->traj_problem.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, st));
+        AS_CUDA(cudaMemcpyAsync(A.us.p, s->traj_off.data(), sizeof(long long) * nt, cudaMemcpyHostToDevice, st));
+        AS_CUDA(cudaMemcpyAsync(A.uw.p, uw.data(), sizeof(long long) * nt, cudaMemcpyHostToDevice, st));
+        AS_CUDA(cudaStreamSynchronize(st));  // the host vectors may go
+        A.traj = s->traj_problem;
+    }
+    if (weights) {
+        AS_CUDA(A.w.alloc(sizeof(double) * (size_t)std::max<long long>(wtot, 1)));
+        AS_CUDA(cudaMemcpyAsync(A.w.p, weights, sizeof(double) * wtot, cudaMemcpyHostToDevice, st));
+    }
+    // A first guess of 48 checkpoints per trajectory; the forward pass counts what it needs.
+    if (!A.ck.p) AS_CUDA(A.ck.alloc(vb * (size_t)std::min<long long>(etot * std::min(max_steps + 1, 48), 1ll << 27)));
 
     AdjointParams P;
     P.inst = s->pool.inst.as<DevInstance>();
-    P.unit_inst = d_ui.as<int>();
-    P.unit_state = d_us.as<long long>();
-    P.unit_wofs = d_uw.as<long long>();
+    P.unit_inst = A.ui.as<int>();
+    P.unit_state = A.us.as<long long>();
+    P.unit_wofs = A.uw.as<long long>();
     P.x0 = s->states.p;
-    P.weights = weights ? d_w.as<double>() : nullptr;
-    P.hs = d_hs.as<double>();
-    P.nsteps = d_ns.as<int>();
-    P.ckpt = nullptr;
-    P.unit_ckpt = nullptr;
-    P.loss = d_loss.as<double>();
-    P.grad_x0 = d_gx.p;
-    P.grad_w = d_gw.as<double>();
+    P.weights = weights ? A.w.as<double>() : nullptr;
+    P.hs = A.hs.as<double>();
+    P.nsteps = A.ns.as<int>();
+    P.ckpt_used = A.used.as<unsigned long long>();
+    P.ckpt_off = A.off.as<long long>();
+    P.loss = A.loss.as<double>();
+    P.grad_x0 = A.gx.p;
+    P.grad_w = A.gw.as<double>();
     P.num_units = nt;
     P.max_steps = max_steps;
     P.eps = s->eps;
     P.t_end = t_end;
 
-    auto launch = [&](AdjFn fn) -> int {
+    int per_sm = 0;
+    AS_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
+    auto launch = [&](AdjFn fn, size_t vals) -> int {
+        const size_t smem = vals * vb;
+        const int bt = adjoint_threads(smem, mmax, nt, s->sm_count, per_sm);
         AS_CUDA(raise_smem_limit((const void*)fn, smem));
         int occ = 0;
         AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, bt, smem));
         if (occ < 1) return fail(AS_ERR_UNSUPPORTED, "adjoint launch shape does not fit on an SM");
         void* args[] = {&P};
-        AS_CUDA(cudaLaunchKernel((const void*)fn, dim3(std::min(nt, s->sm_count * occ)), dim3(bt), args, smem,
-                                 s->stream));
-        AS_CUDA(cudaStreamSynchronize(s->stream));
+        AS_CUDA(cudaLaunchKernel((const void*)fn, dim3(std::min(nt, s->sm_count * occ)), dim3(bt), args, smem, st));
         return AS_OK;
     };
-    int r = launch(av->fwd);
-    if (r) return r;
     std::vector<int> ns(nt);
-    AS_CUDA(cudaMemcpy(ns.data(), d_ns.p, sizeof(int) * nt, cudaMemcpyDeviceToHost));
-    std::vector<long long> uc(nt);
-    long long ctot = 0;
-    for (int t = 0; t < nt; t++) {
-        if (ns[t] < 0)
-            return fail(AS_ERR_UNSUPPORTED, ns[t] == -1 ? "adjoint: more than max_steps steps to reach t_end"
-                                                        : "adjoint: step size underflow");
-        uc[t] = ctot;
-        ctot += (long long)ns[t] * (s->problems[s->traj_problem[t]].n + s->problems[s->traj_problem[t]].m);
+    while (true) {
+        P.ckpt = A.ck.p;
+        P.ckpt_cap = (long long)(A.ck.bytes / vb);
+        AS_CUDA(cudaMemsetAsync(A.ns.p, 0, sizeof(int) * (nt + 2), st));
+        AS_CUDA(cudaMemsetAsync(A.used.p, 0, sizeof(unsigned long long), st));
+        const int r = launch(av->fwd, fvals);
+        if (r) return r;
+        unsigned long long used = 0;
+        AS_CUDA(cudaMemcpyAsync(ns.data(), A.ns.p, sizeof(int) * nt, cudaMemcpyDeviceToHost, st));
+        AS_CUDA(cudaMemcpyAsync(&used, A.used.p, sizeof used, cudaMemcpyDeviceToHost, st));
+        AS_CUDA(cudaStreamSynchronize(st));
+        for (int t = 0; t < nt; t++)
+            if (ns[t] < 0)
+                return fail(AS_ERR_UNSUPPORTED, ns[t] == -1 ? "adjoint: more than max_steps steps to reach t_end"
+                                                            : "adjoint: step size underflow");
+        if ((long long)used <= P.ckpt_cap) break;
+        AS_CUDA(A.ck.alloc(vb * (size_t)used));  // the same steps again, with room for them all
     }
-    AS_CUDA(d_uc.alloc(sizeof(long long) * nt));
-    AS_CUDA(d_ck.alloc(vb * (size_t)std::max<long long>(ctot, 1)));
-    AS_CUDA(cudaMemcpy(d_uc.p, uc.data(), sizeof(long long) * nt, cudaMemcpyHostToDevice));
-    P.ckpt = d_ck.p;
-    P.unit_ckpt = d_uc.as<long long>();
-    r = launch(av->bwd);
+    int r = launch(av->bwd, bvals);
     if (r) return r;
-    AS_CUDA(cudaMemcpy(loss, d_loss.p, sizeof(double) * nt, cudaMemcpyDeviceToHost));
-    AS_CUDA(cudaMemcpy(grad_w, d_gw.p, sizeof(double) * wtot, cudaMemcpyDeviceToHost));
+    AS_CUDA(cudaMemcpyAsync(loss, A.loss.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
+    AS_CUDA(cudaMemcpyAsync(grad_w, A.gw.p, sizeof(double) * wtot, cudaMemcpyDeviceToHost, st));
+    std::vector<float> tmp;
     if (vb == 8) {
-        AS_CUDA(cudaMemcpy(grad_x0, d_gx.p, 8 * (size_t)s->total_values, cudaMemcpyDeviceToHost));
+        AS_CUDA(cudaMemcpyAsync(grad_x0, A.gx.p, 8 * (size_t)s->total_values, cudaMemcpyDeviceToHost, st));
     } else {
-        std::vector<float> tmp((size_t)s->total_values);
-        AS_CUDA(cudaMemcpy(tmp.data(), d_gx.p, 4 * tmp.size(), cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < tmp.size(); i++) grad_x0[i] = tmp[i];
+        tmp.resize((size_t)s->total_values);
+        AS_CUDA(cudaMemcpyAsync(tmp.data(), A.gx.p, 4 * tmp.size(), cudaMemcpyDeviceToHost, st));
     }
+    // the recorded steps: the columns in use, gathered on the device
+    std::vector<double> hs;
+    const int used_steps = *std::max_element(ns.begin(), ns.end());
+    if (step_sizes && used_steps > 0) {
+        const size_t row = sizeof(double) * used_steps;
+        AS_CUDA(A.hsc.alloc(row * nt));
+        AS_CUDA(cudaMemcpy2DAsync(A.hsc.p, row, A.hs.p, sizeof(double) * max_steps, row, nt, cudaMemcpyDeviceToDevice, st));
+        hs.resize((size_t)nt * used_steps);
+        AS_CUDA(cudaMemcpyAsync(hs.data(), A.hsc.p, row * nt, cudaMemcpyDeviceToHost, st));
+    }
+    AS_CUDA(cudaStreamSynchronize(st));
+    for (size_t i = 0; i < tmp.size(); i++) grad_x0[i] = tmp[i];
     if (nsteps) std::copy(ns.begin(), ns.end(), nsteps);
-    if (step_sizes)
-        AS_CUDA(cudaMemcpy(step_sizes, d_hs.p, sizeof(double) * (size_t)nt * max_steps, cudaMemcpyDeviceToHost));
+    if (!hs.empty())
+        for (int t = 0; t < nt; t++)
+            std::copy_n(hs.begin() + (size_t)t * used_steps, ns[t], step_sizes + (size_t)t * max_steps);
+    A.trim();
     return AS_OK;
 }

@@ -115,3 +115,45 @@ def test_adjoint_config4_shape_64_directions(oracle):
         assert _rel(a, b) <= 1e-5, (key, _rel(a, b))
         per = np.array([_rel(a[t * size:(t + 1) * size], b[t * size:(t + 1) * size]) for t in range(P)])
         assert np.quantile(per, 0.99) <= 5e-4, (key, np.quantile(per, 0.99))
+
+
+@pytest.mark.parametrize("precision,tol", [(1, 1e-9), (0, 5e-4)])
+@pytest.mark.parametrize("n,m,lens,starts", [(5, 9, [1, 2, 3], 1), (40, 170, [3], 150), (33, 300, [4], 3),
+                                             (60, 240, [2, 5], 2), (20, 100, [12, 3], 2), (250, 1025, [3], 2)])
+def test_adjoint_shapes_match_oracle(oracle, precision, tol, n, m, lens, starts):
+    """Clause lengths, remainders of the CTA and one to many units per SM, with and without
+    weights; a second call reuses the solver's buffers."""
+    from analogsat_b200 import SatProblem, SatSolver
+    rng = np.random.default_rng(n)
+    length = rng.choice(lens, m)
+    length[0] = max(lens)
+    lits = np.concatenate([(rng.choice(n, k, replace=False) + 1) * rng.choice([-1, 1], k) for k in length])
+    p = SatProblem.from_arrays(lits, length)
+    s = SatSolver([p], precision=precision)
+    s.SetEpsilon(1e-6)
+    dt = np.float32 if precision == 0 else np.float64
+    X = np.ones((starts, p.n + p.m), dt)
+    X[:, : p.n] = rng.uniform(-1, 1, (starts, p.n))
+    s.SetSatStates(np.zeros(starts, np.int32), X)
+    op = oracle.problem(lits, length)
+    E = p.n + p.m
+    for w in (rng.uniform(0.5, 1.5, starts * p.m), None):
+        g = s.Adjoint(2.0, weights=w)
+        for t in {0, starts - 1}:
+            wt = np.ones(p.m) if w is None else w[t * p.m:(t + 1) * p.m]
+            L, gx, gw = oracle.adjoint(op, X[t].astype(np.float64), g["step_sizes"][t], wt)
+            assert abs(g["loss"][t] - L) <= tol * abs(L)
+            assert _rel(g["grad_x0"][t * E:(t + 1) * E], gx) <= tol
+            assert _rel(g["grad_w"][t * p.m:(t + 1) * p.m], gw) <= tol
+
+
+def test_adjoint_checkpoint_pool_grows():
+    """More steps than the first guess of the checkpoint pool holds: the forward pass is
+    repeated with room for all, with the gradients of a call that had the room at once."""
+    s, raw, X, w = _setup(1, P=2)
+    s.SetEpsilon(1e-9)
+    a = s.Adjoint(5.0, weights=w)
+    assert a["nsteps"].min() > 60
+    b = s.Adjoint(5.0, weights=w)
+    for key in ("loss", "grad_x0", "grad_w"):
+        assert np.array_equal(a[key], b[key])
