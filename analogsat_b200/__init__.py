@@ -273,7 +273,7 @@ class SatSolver:
         check(self._lib.as_solver_force_threads(self._h, int(threads)))
 
     def SetKernel(self, kernel: int):
-        """Shared-memory solver kernel: _abi.AS_KERNEL_AUTO (the lean FP32 kernel where the
+        """Shared-memory solver kernel: _abi.AS_KERNEL_AUTO (the lean kernel where the
         instance qualifies) or _abi.AS_KERNEL_GENERIC."""
         check(self._lib.as_solver_set_kernel(self._h, int(kernel)))
 

@@ -188,7 +188,6 @@ struct DevicePool {
                 d.flit = fo >= 0 ? flit.as<uint32_t>() + fo : nullptr;
                 d.cs_off = L.cs_off;
                 d.rows_off = L.rows_off;
-                d.cs_off_g = L.cs_off_g;
                 const size_t i = host_inst.size();
                 const PartLayout* PL = parts && i < parts->size() ? &(*parts)[i] : nullptr;
                 d.nparts = PL ? PL->nparts : 0;
@@ -252,13 +251,16 @@ struct Variant {
     Variant{AS_PREC_F64, K, EX, GS, CL, &solve_kernel<double, false, K, EX, GS, CL>, 8}
 
 #define AS_VARIANT_LEAN(K) \
-    Variant{AS_PREC_F32_LOGA, K, true, false, 1, &solve_kernel_fast<K, false>, 4, true}
+    Variant{AS_PREC_F32_LOGA, K, true, false, 1, &solve_kernel_fast<float, K, false>, 4, true}
 #define AS_VARIANT_LEAN_G(K) \
-    Variant{AS_PREC_F32_LOGA, K, true, true, 1, &solve_kernel_fast<K, true>, 4, true}
+    Variant{AS_PREC_F32_LOGA, K, true, true, 1, &solve_kernel_fast<float, K, true>, 4, true}
+#define AS_VARIANT_LEAN_F64(K, G) \
+    Variant{AS_PREC_F64, K, true, G, 1, &solve_kernel_fast<double, K, G>, 8, true}
 
 const std::vector<Variant>& variants() {
     static const std::vector<Variant> v = {
         AS_VARIANT_LEAN(3), AS_VARIANT_LEAN(4), AS_VARIANT_LEAN_G(3), AS_VARIANT_LEAN_G(4),
+        AS_VARIANT_LEAN_F64(3, false), AS_VARIANT_LEAN_F64(4, false), AS_VARIANT_LEAN_F64(3, true), AS_VARIANT_LEAN_F64(4, true),
         AS_VARIANT_F32(3, true, false, 1),  AS_VARIANT_F32(4, true, false, 1), AS_VARIANT_F32(2, true, false, 1),
         AS_VARIANT_F32(16, false, false, 1), AS_VARIANT_F64(3, true, false, 1), AS_VARIANT_F64(4, true, false, 1),
         AS_VARIANT_F64(16, false, false, 1), AS_VARIANT_F32(3, true, true, 1),  AS_VARIANT_F32(4, true, true, 1),
@@ -269,10 +271,17 @@ const std::vector<Variant>& variants() {
     return v;
 }
 
+// Values of the RK rows, blocked by 32 elements, clauses from the next block.
+size_t lean_row_values(const PackedProblem& q) {
+    return 6 * (size_t)(row_clause_base<true>(q.n) + ((q.m + 31) & ~31));
+}
+
 size_t solver_smem(const Variant& v, const PackedProblem& q) {
     if (v.lean) {
-        const FastLayout L = fast_layout(q.n, q.m, q.nslots);
-        return v.gs ? (size_t)L.cs_off_g + 4 * (size_t)(q.lean_part_slots + 1) : L.bytes;
+        const int vb = (int)v.bytes_per_value;
+        if (v.gs) return (size_t)slots_offset(q.n, vb) + (size_t)vb * (q.lean_part_slots + 1);
+        if (vb == 8) return (size_t)rows_offset(q.n, q.lean_part_slots, vb) + vb * lean_row_values(q);
+        return fast_layout(q.n, q.m, q.nslots).bytes;
     }
     if (v.gs) return 0;
     return solve_smem_values(q.n, q.m, q.nslots) * v.bytes_per_value;
@@ -281,8 +290,7 @@ size_t solver_smem(const Variant& v, const PackedProblem& q) {
 // Values of a trajectory's per-CTA global slab (global-storage variants).
 size_t solver_slab_values(const Variant& v, const PackedProblem& q) {
     if (!v.gs) return 0;
-    if (v.lean)  // the RK rows, blocked by 32 elements, clauses from the next block
-        return 6 * (size_t)(row_clause_base<true>(q.n) + ((q.m + 31) & ~31));
+    if (v.lean) return lean_row_values(q);
     return solve_smem_values(q.n, q.m, q.nslots);
 }
 
@@ -292,7 +300,8 @@ size_t solver_slab_values(const Variant& v, const PackedProblem& q) {
 bool fits(const Variant& v, const PackedProblem& q, int precision, size_t smem_limit) {
     const bool kok = v.exact ? q.k == v.kmax : q.k <= v.kmax;
     if (v.precision != precision || !kok) return false;
-    if (v.lean && v.gs) return standard_model(q) && q.lean_parts > 0 && solver_smem(v, q) <= smem_limit;
+    if (v.lean && (v.gs || precision == AS_PREC_F64))
+        return standard_model(q) && q.lean_parts > 0 && solver_smem(v, q) <= smem_limit;
     if (v.lean) return standard_model(q) && q.compact && fast_layout(q.n, q.m, q.nslots).ok &&
                        solver_smem(v, q) <= smem_limit;
     if (v.gs) return true;
@@ -892,27 +901,31 @@ int32_t as_solver_create(const as_problem* const* problems, int32_t num_problems
     AS_CUDA(cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device));
     AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     s->smem_limit = (size_t)optin - 1024;  // static shared memory of the kernel
-    // FP32 plain-CTDS instances beyond the all-shared lean layout: clause parts for the
-    // lean kernel's global-rows form, the fewest parts whose slots fit one SM
+    // Plain-CTDS instances beyond the FP32 all-shared lean layout: clause parts for the
+    // lean kernel's global-rows form, the fewest parts whose slots fit one SM.  FP64: one
+    // part (the packing itself, literals in the reference's order) where its slots fit.
     s->parts.assign(num_problems, PartLayout());
-    if (precision == AS_PREC_F32_LOGA)
-        for (int i = 0; i < num_problems; i++) {
-            auto& q = s->problems[i];
-            if (!standard_model(q) || (q.k != 3 && q.k != 4) || q.n >= 8191) continue;
+    const bool f64 = precision == AS_PREC_F64;
+    for (int i = 0; i < num_problems; i++) {
+        auto& q = s->problems[i];
+        if (!standard_model(q) || (q.k != 3 && q.k != 4) || q.n >= 8191) continue;
+        if (!f64) {
             const FastLayout L = fast_layout(q.n, q.m, q.nslots);
             if (q.compact && L.ok && L.bytes <= s->smem_limit) continue;  // the all-shared form takes it
-            const HostProblem& hp = problems[i]->host;
-            for (int np = 1; np <= 4; np++) {
-                PartLayout PL;
-                if (!pack_parts(hp, q, np, PL)) break;
-                if ((size_t)L.cs_off_g + 4 * (size_t)(PL.max_slots + 1) <= s->smem_limit) {
-                    q.lean_parts = np;
-                    q.lean_part_slots = PL.max_slots;
-                    s->parts[i] = std::move(PL);
-                    break;
-                }
+        }
+        const int vb = f64 ? 8 : 4;
+        const HostProblem& hp = problems[i]->host;
+        for (int np = 1; np <= (f64 ? 1 : 4); np++) {
+            PartLayout PL;
+            if (!pack_parts(hp, q, np, PL)) break;
+            if ((size_t)slots_offset(q.n, vb) + (size_t)vb * (PL.max_slots + 1) <= s->smem_limit) {
+                q.lean_parts = np;
+                q.lean_part_slots = PL.max_slots;
+                s->parts[i] = std::move(PL);
+                break;
             }
         }
+    }
     std::vector<const PackedProblem*> pk;
     for (auto& q : s->problems) pk.push_back(&q);
     r = s->pool.upload(pk, s->device, &s->parts);

@@ -1,4 +1,4 @@
-// Lean FP32 persistent solver (shared-memory mode, plain CTDS right-hand side).
+// Lean persistent solver (plain CTDS right-hand side): FP32 with log-space weights, and FP64.
 //
 // The same integrator, counters and early-exit rules as solve_kernel (SatSolver::DoSolve
 // + CpuRungeKutta::Step/rkqs/rkck + CpuSat::GetDerivatives/GetClauseViolationCount:
@@ -38,6 +38,13 @@
 //    clauses in parts (each part's contributions summed before the next part reuses
 //    the slots) this takes instances up to N < 8191, where the all-shared layout
 //    stops at N of about 1,240.
+//  * FP64 (the reference's precision): the parts form's words and code with one part,
+//    the rows in shared memory where they fit (N up to about 600 at alpha 4.25) and in the
+//    slab otherwise, every operation rounded in the general kernel's order (bit-identical
+//    results).  The general kernel has to put a whole trajectory beyond N of about 600
+//    -- spins and slots too -- into global memory and takes two words per literal: 256
+//    trajectories of N = 1000, M = 4250, 100 steps took 18.4 ms with it, 6.75 ms here.
+//    Bound by issue and, beyond N of about 600, the L2 latency of the rows.
 // The bank-aware clause grouping of the FP32 packing applies unchanged: a literal's
 // spin and its slot both sit in bank (internal variable mod 32).
 #pragma once
@@ -50,15 +57,14 @@ namespace asb {
 
 // Shared-memory byte offsets of the lean layout for an instance, and whether its
 // literal words can carry them (spin offsets below 16 KB, slot indices below 2^17).
-// bytes: shared memory of the all-shared form (rows on chip); cs_off_g: where the
-// global-rows form's slots start (one spin copy).
+// bytes: shared memory of the all-shared form (rows on chip).
 // The all-shared form holds the spins twice, s_0..s_N (s_N the sentinel) and, from the
 // next multiple of 32 floats (neg_spin_base, so -s_v sits in s_v's bank), -s_0..-s_N: a
 // negated literal's word points at its negated spin and a gather needs no sign flip.
 // Both copies sit at a shared address aligned to spin_align (the smallest power of two
 // >= their bytes), so a spin's address is that base OR the byte offset of its literal
-// word: one logic operation.  bytes counts the worst-case padding.  The global-rows
-// form holds one copy; its slots start at cs_off_g.
+// word: one logic operation.  bytes counts the worst-case padding.  The parts forms hold
+// one copy (slots_offset).
 __host__ __device__ inline int neg_spin_base(int n) { return (n + 1 + 31) & ~31; }
 __host__ __device__ inline uint32_t spin_align(int n) {
     uint32_t a = 128;
@@ -67,13 +73,18 @@ __host__ __device__ inline uint32_t spin_align(int n) {
 }
 struct FastLayout {
     bool ok = false;
-    int cs_off = 0, rows_off = 0, cs_off_g = 0;
+    int cs_off = 0, rows_off = 0;
     size_t bytes = 0;
 };
+// The parts forms (FP32 global rows, FP64): one spin copy, the slots behind it, and behind
+// those (FP64 all in shared memory) the rows.
+__host__ __device__ inline int slots_offset(int n, int vb) { return (vb * (n + 1) + 127) / 128 * 128; }
+__host__ __device__ inline int rows_offset(int n, int part_slots, int vb) {
+    return slots_offset(n, vb) + (vb * (part_slots + 1) + 255) / 256 * 256;
+}
 __host__ __device__ inline FastLayout fast_layout(int n, int m, int nslots) {
     FastLayout L;
     L.cs_off = ((4 * (neg_spin_base(n) + n + 1)) + 127) / 128 * 128;  // a multiple of 128 B keeps slot banks
-    L.cs_off_g = ((4 * (n + 1)) + 127) / 128 * 128;
     const long long cs_end = (long long)L.cs_off + 4ll * (nslots + 1);
     L.rows_off = (int)((cs_end + 15) / 16 * 16);
     L.bytes = (size_t)L.rows_off + 24ull * (size_t)(n + m) + spin_align(n) - 16;
@@ -102,6 +113,11 @@ __device__ __forceinline__ float lds(uint32_t a) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
     return v;
 }
+__device__ __forceinline__ double lds64(uint32_t a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
 __device__ __forceinline__ float2 lds2(uint32_t a) {
     float2 v;
     asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
@@ -110,17 +126,26 @@ __device__ __forceinline__ float2 lds2(uint32_t a) {
 __device__ __forceinline__ void sts(uint32_t a, float v) {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+__device__ __forceinline__ void sts(uint32_t a, double v) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+template <typename T> __device__ __forceinline__ T lds_t(uint32_t a) {
+    if constexpr (sizeof(T) == 4) return lds(a);
+    else return lds64(a);
+}
 
-// The entries of one element's interleaved row that stage S reads (X, K1..K_{S-1}),
-// in 64-bit loads.
+// The entries of one element's row that stage S reads (X, K1..K_{S-1}).
+template <typename T>
 struct Row6 {
-    float x = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f, k4 = 0.f, k5 = 0.f;
+    T x = T(0), k1 = T(0), k2 = T(0), k3 = T(0), k4 = T(0), k5 = T(0);
 };
-// Where the interleaved rows live: shared memory (32-bit shared-window addresses) or a
-// per-CTA global slab.  at(e) is element e's row; ld/ld2/st take the float index in it.
-template <bool G> struct RowStore;
-template <> struct RowStore<false> {
+template <typename T> struct Pair2 { T x, y; };
+// Where the rows live: shared memory (32-bit shared-window addresses) or a per-CTA global
+// slab.  at(e) is element e's row; ld/ld2/st take the field's index in it.
+template <typename T, bool G> struct RowStore;
+template <> struct RowStore<float, false> {
     using Ref = uint32_t;
+    using Val = float;
     uint32_t base;
     __device__ __forceinline__ Ref at(int e) const { return base + 24u * (uint32_t)e; }
     __device__ __forceinline__ static Ref advance(Ref r, int elems) { return r + 24u * (uint32_t)elems; }
@@ -128,40 +153,54 @@ template <> struct RowStore<false> {
     __device__ __forceinline__ static float2 ld2(Ref r, int i) { return lds2(r + 4u * i); }
     __device__ __forceinline__ static void st(Ref r, int i, float v) { sts(r + 4u * i, v); }
 };
+// FP64 rows in shared memory are blocked like those in global memory: a warp's 64-bit
+// accesses to one field are consecutive (at an interleaved 48-byte stride they would
+// take each bank twice).
+template <> struct RowStore<double, false> {
+    using Ref = uint32_t;
+    using Val = double;
+    uint32_t base;
+    __device__ __forceinline__ Ref at(int e) const { return base + 1536u * (uint32_t)(e >> 5) + 8u * (uint32_t)(e & 31); }
+    __device__ __forceinline__ static Ref advance(Ref r, int elems) { return r + 48u * (uint32_t)elems; }
+    __device__ __forceinline__ static double ld(Ref r, int i) { return lds64(r + 256u * i); }
+    __device__ __forceinline__ static Pair2<double> ld2(Ref r, int i) { return {ld(r, i), ld(r, i + 1)}; }
+    __device__ __forceinline__ static void st(Ref r, int i, double v) { sts(r + 256u * i, v); }
+};
 // In global memory the rows are blocked by 32 elements, [e / 32][X, K1..K5][e % 32]: a
-// warp's 32 consecutive elements read or write one field as one 128-byte line (an
-// interleaved 24-byte row would spread a warp's 32-bit store over 24 sectors).
+// warp's 32 consecutive elements read or write one field as one (FP64: two) 128-byte
+// lines (an interleaved 24-byte row would spread a warp's 32-bit store over 24 sectors).
 // advance() takes a multiple of 32 elements.
-template <> struct RowStore<true> {
-    using Ref = float*;
-    float* base;
+template <typename T> struct RowStore<T, true> {
+    using Ref = T*;
+    using Val = T;
+    T* base;
     __device__ __forceinline__ Ref at(int e) const { return base + 192ll * (e >> 5) + (e & 31); }
     __device__ __forceinline__ static Ref advance(Ref r, int elems) { return r + 6ll * elems; }
-    __device__ __forceinline__ static float ld(Ref r, int i) { return r[32 * i]; }
-    __device__ __forceinline__ static float2 ld2(Ref r, int i) { return make_float2(r[32 * i], r[32 * i + 32]); }
-    __device__ __forceinline__ static void st(Ref r, int i, float v) { r[32 * i] = v; }
+    __device__ __forceinline__ static T ld(Ref r, int i) { return r[32 * i]; }
+    __device__ __forceinline__ static Pair2<T> ld2(Ref r, int i) { return {r[32 * i], r[32 * i + 32]}; }
+    __device__ __forceinline__ static void st(Ref r, int i, T v) { r[32 * i] = v; }
 };
-// First row of the clauses: right after the variables' rows in shared memory; in a
-// global slab at the next 32-element block, so a warp's clause rows share blocks.
-template <bool G>
-__host__ __device__ inline int row_clause_base(int n) { return G ? (n + 31) & ~31 : n; }
+// First row of the clauses: right after the variables' rows in shared memory; where rows
+// are blocked at the next 32-element block, so a warp's clause rows share blocks.
+template <bool BLOCKED>
+__host__ __device__ inline int row_clause_base(int n) { return BLOCKED ? (n + 31) & ~31 : n; }
 
 template <int S, typename R>
-__device__ __forceinline__ Row6 load_row(typename R::Ref r) {
-    Row6 o;
+__device__ __forceinline__ Row6<typename R::Val> load_row(typename R::Ref r) {
+    Row6<typename R::Val> o;
     if constexpr (S == 1) {
         o.x = R::ld(r, 0);
     } else {
-        const float2 a = R::ld2(r, 0);
+        const auto a = R::ld2(r, 0);
         o.x = a.x; o.k1 = a.y;
         if constexpr (S == 3) o.k2 = R::ld(r, 2);
         if constexpr (S >= 4) {
-            const float2 b = R::ld2(r, 2);
+            const auto b = R::ld2(r, 2);
             o.k2 = b.x; o.k3 = b.y;
         }
         if constexpr (S == 5) o.k4 = R::ld(r, 4);
         if constexpr (S == 6) {
-            const float2 c = R::ld2(r, 4);
+            const auto c = R::ld2(r, 4);
             o.k4 = c.x; o.k5 = c.y;
         }
     }
@@ -171,10 +210,10 @@ __device__ __forceinline__ Row6 load_row(typename R::Ref r) {
 // (the accepted step's copy of the clause rows is done here, by the owning thread,
 // where the row is read anyway).
 template <int S, typename R>
-__device__ __forceinline__ Row6 load_clause_row(typename R::Ref r, bool from_candidate) {
+__device__ __forceinline__ Row6<typename R::Val> load_clause_row(typename R::Ref r, bool from_candidate) {
     if constexpr (S == 1) {
         if (from_candidate) {
-            Row6 o;
+            Row6<typename R::Val> o;
             o.x = R::ld(r, 2);
             R::st(r, 0, o.x);
             return o;
@@ -182,14 +221,14 @@ __device__ __forceinline__ Row6 load_clause_row(typename R::Ref r, bool from_can
     }
     return load_row<S, R>(r);
 }
-template <int S>
-__device__ __forceinline__ float row_input(const Row6& o, float h) {
-    return stage_in<S, float>(o.x, o.k1, o.k2, o.k3, o.k4, o.k5, h);
+template <int S, typename T>
+__device__ __forceinline__ T row_input(const Row6<T>& o, T h) {
+    return stage_in<S, T>(o.x, o.k1, o.k2, o.k3, o.k4, o.k5, h);
 }
 // Puts the stage-S derivative into its place of a row read for stage S, which then
 // holds what stage S + 1 reads.
-template <int S>
-__device__ __forceinline__ void set_k(Row6& o, float k) {
+template <int S, typename T>
+__device__ __forceinline__ void set_k(Row6<T>& o, T k) {
     if constexpr (S == 1) o.k1 = k;
     if constexpr (S == 2) o.k2 = k;
     if constexpr (S == 3) o.k3 = k;
@@ -273,6 +312,42 @@ __device__ __forceinline__ float part_clause(uint32_t sm0, uint32_t cs0, const u
     return (P * P) * duc;
 }
 
+// FP64, linear weights: every operation rounded as clause_phase<double, false> rounds it
+// (the reference's order), so the results are bit-identical; returns da_m.
+template <int K>
+__device__ __forceinline__ double part_clause(uint32_t sm0, uint32_t cs0, const uint32_t* lp, double am,
+                                              double knorm) {
+    auto flip = [](double a, uint32_t w) {  // -a for a negated literal
+        return __hiloint2double(__double2hiint(a) ^ (int)(w & 0x80000000u), __double2loint(a));
+    };
+    uint32_t w[K];
+    double f[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) w[q] = ld_lit(lp + 32 * q);
+    double km = knorm;
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        f[q] = __dsub_rn(1.0, flip(lds64(sm0 + 8u * (w[q] & 0x1FFFu)), w[q]));
+        km = __dmul_rn(km, f[q]);
+    }
+    const double r = __dmul_rn(__dmul_rn(km, knorm), am);
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        double prod = 1.0;
+        bool first = true;
+#pragma unroll
+        for (int l = 0; l < K; l++) {
+            if (l != q) {
+                prod = first ? f[l] : __dmul_rn(prod, f[l]);
+                first = false;
+            }
+        }
+        const double rr = __dmul_rn(r, prod);
+        sts(cs0 + 8u * ((w[q] >> 13) & 0x1FFFFu), flip(__dadd_rn(rr, rr), w[q]));
+    }
+    return __dmul_rn(__dmul_rn(am, km), km);
+}
+
 // Block max of the error ratios, post-processed by thread 0.  The ratios are FP32 and
 // never negative (fmaxf from 0 skips NaN), so their bit patterns order like their values
 // and a warp's max is one integer redux; the max of floats then converted is the FP64
@@ -292,18 +367,39 @@ __device__ __forceinline__ double lean_max_then(float em, uint32_t* red_u, doubl
     return red_d[33];
 }
 
+template <typename F>
+__device__ __forceinline__ double lean_max_then(double em, uint32_t*, double* red_d, F&& fn) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) red_d[warp] = em;
+    __syncthreads();
+    if (warp == 0) {
+        double x = lane < (int)(blockDim.x >> 5) ? red_d[lane] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+        if (lane == 0) red_d[33] = fn(x);
+    }
+    __syncthreads();
+    return red_d[33];
+}
+
 __device__ __forceinline__ int ld_relaxed(const int* p) {
     int v;
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
-// ROWS_G = false: rows, spins and slots in shared memory, words flit.  ROWS_G = true:
+// FP32, ROWS_G = false: rows, spins and slots in shared memory, words flit.  ROWS_G = true:
 // rows in the CTA's global slab, spins and slots in shared memory, clauses in parts
 // (words plit), each part's contributions summed before the next part reuses the slots.
-template <int K, bool ROWS_G>
+// FP64: words plit in one part, rows in shared memory or the slab.
+template <typename T, int K, bool ROWS_G>
 __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
-    using R = RowStore<ROWS_G>;
+    using R = RowStore<T, ROWS_G>;
+    constexpr bool LOGA = sizeof(T) == 4;              // a_m held as log2 a_m
+    constexpr bool PARTS = ROWS_G || sizeof(T) == 8;   // words plit, rows blocked by 32
+    constexpr uint32_t VB = (uint32_t)sizeof(T);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red_d[36];
     __shared__ int red_i[33];
@@ -329,37 +425,47 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
             continue;
         }
         const DevInstance I = P.inst[pidx];
-        const int n = I.n, m = I.m, cb = row_clause_base<ROWS_G>(n);
+        const int n = I.n, m = I.m, cb = row_clause_base<PARTS>(n);
         // spin base: aligned in the all-shared form (spin_align), the start otherwise
-        const uint32_t mask = ROWS_G ? 0u : spin_align(n) - 1u;
-        const uint32_t sb = ROWS_G ? sm0 : (sm0 + mask) & ~mask;
-        float* const sy = reinterpret_cast<float*>(smem_raw + (sb - sm0));
-        const int cso = ROWS_G ? I.cs_off_g : I.cs_off;
-        float* const cs = reinterpret_cast<float*>(smem_raw + (sb - sm0) + cso);
+        const uint32_t mask = PARTS ? 0u : spin_align(n) - 1u;
+        const uint32_t sb = PARTS ? sm0 : (sm0 + mask) & ~mask;
+        T* const sy = reinterpret_cast<T*>(smem_raw + (sb - sm0));
+        const int cso = PARTS ? slots_offset(n, VB) : I.cs_off;
+        T* const cs = reinterpret_cast<T*>(smem_raw + (sb - sm0) + cso);
         R rs;
-        if constexpr (ROWS_G) rs.base = reinterpret_cast<float*>(P.slab) + (long long)blockIdx.x * P.slab_stride;
+        if constexpr (ROWS_G) rs.base = reinterpret_cast<T*>(P.slab) + (long long)blockIdx.x * P.slab_stride;
+        else if constexpr (PARTS) rs.base = sb + (uint32_t)rows_offset(n, I.part_slots, VB);
         else rs.base = sb + (uint32_t)I.rows_off;
         const uint32_t cs0 = sb + (uint32_t)cso;
         // the all-shared form's second, negated spin copy: spin v also at sneg + 4 v
         const uint32_t sneg = sb + 4u * (uint32_t)neg_spin_base(n);
-        auto put_spin = [&](int v, float val) {
-            sts(sb + 4u * (uint32_t)v, val);
-            if constexpr (!ROWS_G) sts(sneg + 4u * (uint32_t)v, -val);
+        auto put_spin = [&](int v, T val) {
+            sts(sb + VB * (uint32_t)v, val);
+            if constexpr (!PARTS) sts(sneg + 4u * (uint32_t)v, -val);
         };
-        float* G = reinterpret_cast<float*>(P.states) + P.unit_state[u];
-        const float knorm = (float)ldexp(1.0, -I.k);
-        const float a2n = 2.0f * knorm * knorm;      // 2 knorm^2 (exact)
-        const float duc = knorm * knorm * kInvLn2;   // knorm^2 / ln 2 (exact scaling)
+        T* G = reinterpret_cast<T*>(P.states) + P.unit_state[u];
+        const T knorm = (T)ldexp(1.0, -I.k);
+        // FP32: 2 knorm^2 (exact) and knorm^2 / ln 2 (exact scaling); FP64 scales by knorm itself
+        const T a2n = LOGA ? T(2) * knorm * knorm : T(1);
+        const T duc = LOGA ? knorm * knorm * T(kInvLn2) : knorm;
+        auto weight = [&](T y) {  // a_m (FP32: times a2n) from the stage input
+            if constexpr (LOGA) return exp2_fast(y) * a2n;
+            else return y;
+        };
         // the wall-clock deadline (stamped before the launch)
         const unsigned long long deadline = P.deadline ? *P.deadline : 0ull;
 
         // initial state: public spins to internal order, a -> log2 a
-        const int32_t* const icp = ROWS_G ? I.picperm : I.icperm;  // public -> internal clause
+        const int32_t* const icp = PARTS ? I.picperm : I.icperm;  // public -> internal clause
         for (int i = tid; i < n; i += nt) R::st(rs.at(__ldg(I.iperm + i)), 0, G[i]);
-        for (int j = tid; j < m; j += nt) R::st(rs.at(cb + __ldg(icp + j)), 0, log2f(G[n + j]));
-        if constexpr (!ROWS_G)  // padding slots are read as zeros (the parts form reads counts)
-            for (int j = tid; j <= I.nslots; j += nt) cs[j] = 0.0f;
-        if (tid == 0) put_spin(n, -1.0f);  // sentinel spin: padding literals are always FALSE
+        for (int j = tid; j < m; j += nt) {
+            T a = G[n + j];
+            if constexpr (LOGA) a = log2f(a);
+            R::st(rs.at(cb + __ldg(icp + j)), 0, a);
+        }
+        if constexpr (!PARTS)  // padding slots are read as zeros (the parts form reads counts)
+            for (int j = tid; j <= I.nslots; j += nt) cs[j] = T(0);
+        if (tid == 0) put_spin(n, T(-1));  // sentinel spin: padding literals are always FALSE
         g.sync();  // the scatter above wrote rows that other threads own in the stage loops
 
         // The step size after an accepted step (CpuRungeKutta.cpp:252-256) is needed only
@@ -383,26 +489,26 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
         // for S == 6 is consumed at once into the candidate state (slot 2) and the error
         // norm.  The spins' stage input is formed by the variable phase of the stage
         // before (ready = true; stage 1's by the accepted step's copy), or here.
-        auto eval = [&](auto stage, float hT, float h0T, float& em, bool ready) {
+        auto eval = [&](auto stage, T hT, T h0T, T& em, bool ready) {
             constexpr int S = decltype(stage)::value;
             if (!ready)
                 for (int v = tid; v < n; v += nt)
                     put_spin(v, row_input<S>(load_row<S, R>(rs.at(v)), hT));
             g.sync();
-            if constexpr (ROWS_G) {
+            if constexpr (PARTS) {
                 const int np = I.nparts, ns1 = ((n + 31) >> 5) + 1;
                 for (int pp = 0; pp < np; pp++) {
                     const int c0 = ld_ro(I.part_c0 + pp), c1 = ld_ro(I.part_c0 + pp + 1);
                     const uint32_t* lp = I.plit + lean_word_index(c0 + tid, 0, K);
                     typename R::Ref ra = rs.at(cb + c0 + tid);
                     for (int c = c0 + tid; c < c1; c += nt, lp += (size_t)nt * K, ra = R::advance(ra, nt)) {
-                        const Row6 o = load_clause_row<S, R>(ra, ready);
-                        const float d = part_clause<K>(sb, cs0, lp, exp2_fast(row_input<S>(o, hT)) * a2n, duc);
+                        const auto o = load_clause_row<S, R>(ra, ready);
+                        const T d = part_clause<K>(sb, cs0, lp, weight(row_input<S>(o, hT)), duc);
                         if constexpr (S < 6) {
                             R::st(ra, S, d);
                         } else {
-                            em = fmaxf(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, d, hT, h0T, true));
-                            R::st(ra, 2, rk_new<float>(o.x, o.k1, o.k3, o.k4, d, hT));
+                            em = fmax(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, d, hT, h0T, LOGA));
+                            R::st(ra, 2, rk_new<T>(o.x, o.k1, o.k3, o.k4, d, hT));
                         }
                     }
                     if constexpr (S == 1)
@@ -420,8 +526,8 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                     // L2 latencies overlap.
                     struct VarIn {
                         int cnt, r0;
-                        float sum;
-                        Row6 o;
+                        T sum;
+                        Row6<T> o;
                     };
                     auto var_load = [&](int v) {
                         VarIn a;
@@ -429,26 +535,26 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                         a.r0 = ld_ro(I.part_srow + (size_t)pp * ns1 + (v >> 5));
                         const typename R::Ref r = rs.at(v);
                         if (last) a.o = load_row<S, R>(r);
-                        a.sum = pp == 0 ? 0.0f : R::ld(r, SLOT);
+                        a.sum = pp == 0 ? T(0) : R::ld(r, SLOT);
                         return a;
                     };
                     auto var_sum = [&](int v, const VarIn& a) {
-                        uint32_t pa = cs0 + 4u * (uint32_t)(a.r0 * 32 + (v & 31));
-                        float sum = a.sum;
+                        uint32_t pa = cs0 + VB * (uint32_t)(a.r0 * 32 + (v & 31));
+                        T sum = a.sum;
 #pragma unroll 8
-                        for (int k = 0; k < a.cnt; k++, pa += 128u) sum = sum + lds(pa);
+                        for (int k = 0; k < a.cnt; k++, pa += 32u * VB) sum = Arith<T>::add(sum, lds_t<T>(pa));
                         const typename R::Ref r = rs.at(v);
                         if (!last) {
                             R::st(r, SLOT, sum);
                         } else if constexpr (S < 6) {
-                            Row6 o = a.o;
+                            Row6<T> o = a.o;
                             R::st(r, S, sum);
                             set_k<S>(o, sum);
-                            put_spin(v, row_input<S + 1>(o, S == 1 ? (float)hnext : hT));
+                            put_spin(v, row_input<S + 1>(o, S == 1 ? (T)hnext : hT));
                         } else {
-                            const Row6& o = a.o;
-                            em = fmaxf(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, sum, hT, h0T, false));
-                            R::st(r, 2, rk_new<float>(o.x, o.k1, o.k3, o.k4, sum, hT));
+                            const Row6<T>& o = a.o;
+                            em = fmax(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, sum, hT, h0T, false));
+                            R::st(r, 2, rk_new<T>(o.x, o.k1, o.k3, o.k4, sum, hT));
                         }
                     };
                     for (int v = tid; v < n; v += 2 * nt) {
@@ -466,13 +572,13 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
             const uint32_t* lp = I.flit + lean_word_index(tid, 0, K);
             typename R::Ref ra = rs.at(cb + tid);
             for (int c = tid; c < m; c += nt, lp += (size_t)nt * K, ra = R::advance(ra, nt)) {
-                const Row6 o = load_clause_row<S, R>(ra, ready);
-                const float d = fast_clause<K>(sb, mask, cs0, lp, exp2_fast(row_input<S>(o, hT)) * a2n, duc);
+                const auto o = load_clause_row<S, R>(ra, ready);
+                const T d = fast_clause<K>(sb, mask, cs0, lp, weight(row_input<S>(o, hT)), duc);
                 if constexpr (S < 6) {
                     R::st(ra, S, d);
                 } else {
-                    em = fmaxf(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, d, hT, h0T, true));
-                    R::st(ra, 2, rk_new<float>(o.x, o.k1, o.k3, o.k4, d, hT));
+                    em = fmax(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, d, hT, h0T, LOGA));
+                    R::st(ra, 2, rk_new<T>(o.x, o.k1, o.k3, o.k4, d, hT));
                 }
             }
             if constexpr (S == 1) settle_h();
@@ -483,17 +589,17 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                 const int r0 = ld_ro(I.srow + g32), r1 = ld_ro(I.srow + g32 + 1);
                 uint32_t p = cs0 + 4u * (uint32_t)(r0 * 32 + (v & 31));
                 const typename R::Ref r = rs.at(v);
-                Row6 o = load_row<S, R>(r);  // what the next stage's input (or stage 6) reads
-                float sum = 0.0f;
+                Row6<T> o = load_row<S, R>(r);  // what the next stage's input (or stage 6) reads
+                T sum = T(0);
 #pragma unroll 8
                 for (int k = r0; k < r1; k++, p += 128u) sum = sum + lds(p);
                 if constexpr (S < 6) {
                     R::st(r, S, sum);
                     set_k<S>(o, sum);
-                    put_spin(v, row_input<S + 1>(o, S == 1 ? (float)hnext : hT));
+                    put_spin(v, row_input<S + 1>(o, S == 1 ? (T)hnext : hT));
                 } else {
-                    em = fmaxf(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, sum, hT, h0T, false));
-                    R::st(r, 2, rk_new<float>(o.x, o.k1, o.k3, o.k4, sum, hT));
+                    em = fmax(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, sum, hT, h0T, false));
+                    R::st(r, 2, rk_new<T>(o.x, o.k1, o.k3, o.k4, sum, hT));
                 }
             }
         };
@@ -509,17 +615,17 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
             bool underflow = false, interrupted = false;
             int taken = 0;
             for (int b = 0; b < P.batch; b++) {
-                float dummy = 0.0f;
-                eval(std::integral_constant<int, 1>{}, 0.0f, 0.0f, dummy, s1_ready);
+                T dummy = T(0);
+                eval(std::integral_constant<int, 1>{}, T(0), T(0), dummy, s1_ready);
                 s1_ready = false;  // the clause rows' copy is done
                 rhs++;
                 const double h0 = hnext;
-                const float h0T = (float)h0;
+                const T h0T = (T)h0;
                 double h = hnext, ermax = 0.0;
                 bool retry = false;  // a retry's stage-2 input uses the smaller step
                 while (true) {
-                    const float hT = (float)h;
-                    float em = 0.0f;
+                    const T hT = (T)h;
+                    T em = T(0);
                     eval(std::integral_constant<int, 2>{}, hT, h0T, em, !retry);
                     eval(std::integral_constant<int, 3>{}, hT, h0T, em, true);
                     eval(std::integral_constant<int, 4>{}, hT, h0T, em, true);
@@ -560,7 +666,7 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                 // stage 1's input.  The clause rows follow in that stage's clause loop.
                 for (int v = tid; v < n; v += nt) {
                     const typename R::Ref r = rs.at(v);
-                    const float xn = R::ld(r, 2);
+                    const T xn = R::ld(r, 2);
                     R::st(r, 0, xn);
                     put_spin(v, xn);
                 }
@@ -571,21 +677,21 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
             if (interrupted) { status = SAT_ODE_INTERRUPTED; break; }
 
             // CpuSat::GetClauseViolationCount on the accepted state
-            for (int v = tid; v < n; v += nt) sts(sb + 4u * (uint32_t)v, R::ld(rs.at(v), 0));
+            for (int v = tid; v < n; v += nt) sts(sb + VB * (uint32_t)v, R::ld(rs.at(v), 0));
             g.sync();
             int cnt = 0;
             {
-                const uint32_t* lp = (ROWS_G ? I.plit : I.flit) + lean_word_index(tid, 0, K);
+                const uint32_t* lp = (PARTS ? I.plit : I.flit) + lean_word_index(tid, 0, K);
                 for (int c = tid; c < m; c += nt, lp += (size_t)nt * K) {
                     bool sat = false;
 #pragma unroll
                     for (int q = 0; q < K; q++) {
                         const uint32_t w = ld_lit(lp + 32 * q);
                         // the positive spin (the word of a negated literal points at -s)
-                        const uint32_t sa = ROWS_G ? sb + 4u * (w & 0x1FFFu)
+                        const uint32_t sa = PARTS ? sb + VB * (w & 0x1FFFu)
                                                    : (w & 0x80000000u) ? (sb | (w & mask)) - 4u * (uint32_t)neg_spin_base(n)
                                                                        : (sb | (w & mask));
-                        const bool tv = lds(sa) > 0.0f;
+                        const bool tv = lds_t<T>(sa) > T(0);
                         sat |= (w & 0x80000000u) ? !tv : tv;
                     }
                     cnt += sat ? 0 : 1;
@@ -598,7 +704,7 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                     uint32_t* bits = P.best_bits + P.unit_bits[u];
                     for (int i0 = tid & ~31; i0 < n; i0 += nt) {
                         const int i = i0 + (tid & 31);
-                        const bool bb = i < n && sy[__ldg(I.iperm + (i < n ? i : 0))] > 0.0f;
+                        const bool bb = i < n && sy[__ldg(I.iperm + (i < n ? i : 0))] > T(0);
                         const unsigned bal = __ballot_sync(0xffffffffu, bb);
                         if ((tid & 31) == 0) bits[i0 >> 5] = bal;
                     }
@@ -624,7 +730,11 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
         // write back the final state in the public layout
         g.sync();
         for (int i = tid; i < n; i += nt) G[i] = R::ld(rs.at(__ldg(I.iperm + i)), 0);
-        for (int j = tid; j < m; j += nt) G[n + j] = exp2f(R::ld(rs.at(cb + __ldg(icp + j)), s1_ready ? 2 : 0));
+        for (int j = tid; j < m; j += nt) {
+            const T a = R::ld(rs.at(cb + __ldg(icp + j)), s1_ready ? 2 : 0);
+            if constexpr (LOGA) G[n + j] = exp2f(a);
+            else G[n + j] = a;
+        }
         if (tid == 0) {
             UnitResult r;
             r.time = t; r.hdid = hdid; r.status = status; r.steps = steps; r.attempts = attempts;
