@@ -348,6 +348,18 @@ int shared_cta_threads(size_t smem_bytes, int bt, int device, int* out) {
     return AS_OK;
 }
 
+// CTA size of a group with few units: an SM runs at most `per` of its CTAs, so each takes
+// its share of the SM's 1,024 threads (64 registers each), up to one clause per thread and
+// a warp without clauses for the step size's pow().  Never fewer threads than `bt`, the size
+// for a full GPU.  us per RHS of a trajectory, 16 trajectories, bt threads and so: N = 50
+// FP64 1.55 -> 1.09, FP32 0.89 -> 0.61; N = 200 FP32 1.01 -> 0.89; 300 of N = 50 FP64 1.54 ->
+// 1.17 (before the FP64 redux of the error max).
+int few_units_threads(int bt, int m, int units, int sms) {
+    const int per = (units + sms - 1) / sms;
+    const int share = 1024 / per / 32 * 32, one = (m + 31) / 32 * 32 + 32;
+    return std::max(bt, std::min(share, one));
+}
+
 __global__ void stamp_deadline_kernel(unsigned long long* out, unsigned long long budget_ns) {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1099,11 +1111,12 @@ int build_groups(as_solver* s) {
     for (int u = 0; u < num_traj;) {
         const int vi = pv[pi[s->order[u]]];
         const Variant& v = vs[vi];
-        int e = u, bt = 64;
+        int e = u, bt = 64, mmax = 1;
         size_t vals = 0, sbytes = 0;
         while (e < num_traj && pv[pi[s->order[e]]] == vi) {
             const auto& q = s->problems[pi[s->order[e]]];
             bt = std::max(bt, preferred_bt(q));
+            mmax = std::max(mmax, q.m);
             vals = std::max(vals, solver_slab_values(v, q));
             sbytes = std::max(sbytes, solver_smem(v, q));
             e++;
@@ -1126,6 +1139,7 @@ int build_groups(as_solver* s) {
         if (!v.gs || v.lean) {
             const int r = shared_cta_threads(sbytes, bt, s->device, &sm_bt);
             if (r) return r;
+            sm_bt = few_units_threads(sm_bt, mmax, e - u, s->sm_count);
         }
         G.bt = s->forced_bt ? s->forced_bt : (v.gs && !v.lean ? (v.cl > 1 ? 1024 : gs_bt) : sm_bt);
         G.smem = sbytes;

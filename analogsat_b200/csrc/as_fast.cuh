@@ -367,17 +367,22 @@ __device__ __forceinline__ double lean_max_then(float em, uint32_t* red_u, doubl
     return red_d[33];
 }
 
+// FP64 ratios are never negative either, so their bit patterns order like their values:
+// the high words' max, then the low words' among the lanes that hold it.
+__device__ __forceinline__ double warp_max_bits(double v) {
+    const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+    const uint32_t h = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t l = __reduce_max_sync(0xffffffffu, hi == h ? lo : 0u);
+    return __hiloint2double((int)h, (int)l);
+}
 template <typename F>
 __device__ __forceinline__ double lean_max_then(double em, uint32_t*, double* red_d, F&& fn) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
+    em = warp_max_bits(em);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) red_d[warp] = em;
     __syncthreads();
     if (warp == 0) {
-        double x = lane < (int)(blockDim.x >> 5) ? red_d[lane] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+        const double x = warp_max_bits(lane < (int)(blockDim.x >> 5) ? red_d[lane] : 0.0);
         if (lane == 0) red_d[33] = fn(x);
     }
     __syncthreads();
@@ -471,7 +476,8 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
         // The step size after an accepted step (CpuRungeKutta.cpp:252-256) is needed only
         // from the next step's stage 2 on, so it is formed during the next stage 1, after
         // the clause loop, by lane 0 of the last warp: that warp has no more clauses than
-        // the first, so the FP64 pow() runs while the first warps finish theirs.
+        // the first (none, where the host adds a warp for it), so the FP64 pow() runs while
+        // the first warps do theirs.
         double hnext = 1e-9, e_acc = 0.0, h_acc = 0.0;
         bool h_pending = false;
         const int pow_tid = nt >= 64 ? nt - 32 : 0;
