@@ -169,16 +169,23 @@ class SatProblem:
             pass
 
 
-def _stream_ptr(stream):
+def _stream_handle(stream) -> int:
     """A CUDA stream handle: an int (cudaStream_t), an object with .cuda_stream (a
     torch.cuda.Stream), or None for torch's current stream."""
     if stream is None:
         try:
             import torch
-            return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+            try:  # the handle alone: a Stream object costs a microsecond a call
+                return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+            except AttributeError:
+                return torch.cuda.current_stream().cuda_stream
         except Exception:
-            return C.c_void_p(0)
-    return C.c_void_p(int(getattr(stream, "cuda_stream", stream)))
+            return 0
+    return int(getattr(stream, "cuda_stream", stream))
+
+
+def _stream_ptr(stream):
+    return C.c_void_p(_stream_handle(stream))
 
 
 def get_derivatives(problem: SatProblem, x, out=None, logspace: bool = False, stream=None):
@@ -196,11 +203,9 @@ def get_derivatives(problem: SatProblem, x, out=None, logspace: bool = False, st
     if x.dtype == torch.float64:
         if logspace:
             raise AnalogSatError(_abi.AS_ERR_UNSUPPORTED, "log-space RHS is FP32 only")
-        check(lib.as_rhs_f64(problem._h, C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()), B,
-                             _stream_ptr(stream)))
+        check(lib.as_rhs_f64(problem._h, x.data_ptr(), out.data_ptr(), B, _stream_handle(stream)))
     elif x.dtype == torch.float32:
-        check(lib.as_rhs_f32(problem._h, C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()), B,
-                             int(logspace), _stream_ptr(stream)))
+        check(lib.as_rhs_f32(problem._h, x.data_ptr(), out.data_ptr(), B, int(logspace), _stream_handle(stream)))
     else:
         raise AnalogSatError(_abi.AS_ERR_BAD_INPUT, "x must be float32 or float64")
     return out
@@ -220,8 +225,7 @@ def clause_violation_counts(problem: SatProblem, x, stream=None):
     out = torch.empty(B, dtype=torch.int32, device=x.device)
     lib = load()
     fn = lib.as_violations_f64 if x.dtype == torch.float64 else lib.as_violations_f32
-    check(fn(problem._h, C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()), B,
-             _stream_ptr(stream)))
+    check(fn(problem._h, x.data_ptr(), out.data_ptr(), B, _stream_handle(stream)))
     return out
 
 
@@ -244,7 +248,7 @@ class SatSolver:
         h = C.c_void_p()
         check(self._lib.as_solver_create(arr, len(self.problems), precision, device, C.byref(h)))
         self._h = h
-        self._nm = [(p.n, p.m) for p in self.problems]
+        self._nm = np.array([(p.n, p.m) for p in self.problems], np.int64)
         self._traj_problem = None
 
     # -- configuration (SatSolver.h:133-160, CpuRungeKutta.cpp:126-131) --
@@ -364,9 +368,9 @@ class SatSolver:
     def GetSatStates(self, dtype=np.float64, out=None) -> np.ndarray:
         """Final public states, concatenated (SatSolver::GetSatState().CopyTo).
         `out` may be a preallocated (e.g. pinned) host array of the right size/dtype."""
-        total = int(sum(sum(self._nm[p]) for p in self._traj_problem))
+        total = int(self._nm[self._traj_problem].sum())
         if out is None:
-            out = np.zeros(total, dtype)
+            out = np.empty(total, dtype)
         dtype = out.dtype
         if out.size != total or not out.flags.c_contiguous:
             raise AnalogSatError(_abi.AS_ERR_BAD_INPUT, "out has the wrong size or layout")
@@ -400,28 +404,27 @@ class SatSolver:
         bits = np.zeros((n + 31) // 32, np.uint32)
         check(self._lib.as_solver_get_best_assignment(self._h, int(traj),
                                                       bits.ctypes.data_as(C.c_void_p)))
-        return ((bits[np.arange(n) // 32] >> (np.arange(n) % 32).astype(np.uint32)) & 1).astype(bool)
+        return np.unpackbits(bits.view(np.uint8), count=n, bitorder="little").view(np.bool_)
 
     def Adjoint(self, t_end: float, weights=None, max_steps: int = 4096) -> dict:
         """Gradients of L = sum_m w_m a_m(T) K_m(T)^2 w.r.t. x(0) and w for every
         trajectory (see as_solver_adjoint); x(0) is the current state buffer."""
         nt = len(self._traj_problem)
-        ms = [self._nm[p][1] for p in self._traj_problem]
-        total = int(sum(sum(self._nm[p]) for p in self._traj_problem))
-        loss = np.zeros(nt); gx = np.zeros(total); gw = np.zeros(max(sum(ms), 1))
-        ns = np.zeros(nt, np.int32)
-        hs = np.zeros((nt, max_steps))
+        total, msum = int(self._nm[self._traj_problem].sum()), int(self._nm[self._traj_problem, 1].sum())
+        loss = np.empty(nt); gx = np.empty(total); gw = np.empty(max(msum, 1))
+        ns = np.empty(nt, np.int32)
+        hs = np.empty((nt, max_steps))
         wp = None
         if weights is not None:
             weights = np.ascontiguousarray(weights, np.float64)
-            if weights.size != sum(ms):
+            if weights.size != msum:
                 raise AnalogSatError(_abi.AS_ERR_BAD_INPUT, "weights: M values per trajectory")
             wp = weights.ctypes.data_as(C.c_void_p)
         check(self._lib.as_solver_adjoint(self._h, float(t_end), int(max_steps), wp,
                                           loss.ctypes.data_as(C.c_void_p), gx.ctypes.data_as(C.c_void_p),
                                           gw.ctypes.data_as(C.c_void_p), ns.ctypes.data_as(C.c_void_p),
                                           hs.ctypes.data_as(C.c_void_p)))
-        return dict(loss=loss, grad_x0=gx, grad_w=gw[: sum(ms)], nsteps=ns,
+        return dict(loss=loss, grad_x0=gx, grad_w=gw[:msum], nsteps=ns,
                     step_sizes=[hs[t, : ns[t]].copy() for t in range(nt)])
 
     def kernel_name(self) -> str:

@@ -218,6 +218,28 @@ struct DevicePool {
     }
 };
 
+// What the launch rules read of a device, asked of the driver once per device.
+struct DeviceLimits {
+    int sms = 0, smem_optin = 0, smem_per_sm = 0;
+};
+int device_limits(int dev, DeviceLimits* out) {
+    static std::mutex mu;
+    static std::vector<std::pair<int, DeviceLimits>> known;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const auto& k : known)
+        if (k.first == dev) {
+            *out = k.second;
+            return AS_OK;
+        }
+    DeviceLimits L;
+    AS_CUDA(cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev));
+    AS_CUDA(cudaDeviceGetAttribute(&L.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    AS_CUDA(cudaDeviceGetAttribute(&L.smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    known.emplace_back(dev, L);
+    *out = L;
+    return AS_OK;
+}
+
 int current_device(int requested, int* out) {
     if (requested >= 0) {
         AS_CUDA(cudaSetDevice(requested));
@@ -381,6 +403,10 @@ struct as_problem {
     std::mutex mu_;
     DevicePool dev[3];        // lazily uploaded for the device primitives
     DevBuf slab[3];           // per-CTA storage of the global-storage primitives
+    // Kernels of the standalone primitives that have been prepared for this problem (shared
+    // memory limit raised, occupancy asked): the instance fixes the shape of each.
+    struct Prepared { const void* fn; int dev; size_t smem; int occ; };
+    std::vector<Prepared> prepared_;
     DevBuf rhs_status;        // set by a device RHS whose bulk copy timed out (as_rhs_check)
     int rhs_status_dev = -1;  // device holding rhs_status
 
@@ -425,6 +451,18 @@ constexpr size_t kAdjointKeep = 1ull << 30;
 struct AdjointPlan {
     DevBuf ui, us, uw, w, hs, off, ns, used, loss, gx, gw, ck, hsc;
     std::vector<int> traj;  // the trajectories that ui, us and uw describe
+    float* pinned = nullptr;  // FP32 gradients on their way to the caller's FP64 array
+    size_t pinned_values = 0;
+    ~AdjointPlan() { if (pinned) cudaFreeHost(pinned); }
+    cudaError_t pin(size_t values) {
+        if (values <= pinned_values) return cudaSuccess;
+        if (pinned) cudaFreeHost(pinned);
+        pinned = nullptr;
+        pinned_values = 0;
+        const cudaError_t e = cudaMallocHost(&pinned, values * sizeof(float));
+        if (e == cudaSuccess) pinned_values = values;
+        return e;
+    }
     void trim() {
         for (DevBuf* b : {&ck, &hs, &off})
             if (b->bytes > kAdjointKeep) b->release();
@@ -661,6 +699,21 @@ int32_t as_problem_get_model(const as_problem* p, int32_t* model, double* q, dou
 // ---- device primitives ----
 namespace {
 
+// CTAs per SM of kernel `fn` at this shape, with its shared-memory limit raised to `smem`;
+// asked of the driver on a problem's first call (1 to 2 us each of a call's 9).
+int prepare_kernel(as_problem* p, const void* fn, int bt, size_t smem, int dev, int* occ) {
+    std::lock_guard<std::mutex> lock(p->mu_);
+    for (const auto& k : p->prepared_)
+        if (k.fn == fn && k.dev == dev && k.smem == smem) {
+            *occ = k.occ;
+            return AS_OK;
+        }
+    AS_CUDA(raise_smem_limit(fn, smem));
+    AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, fn, bt, smem));
+    p->prepared_.push_back({fn, dev, smem, *occ});
+    return AS_OK;
+}
+
 int ensure_uploaded(as_problem* p, int prec) {
     if (p->host.m == 0 || p->host.k == 0) return fail(AS_ERR_NO_PROBLEM, "SAT problem has not been set");
     int dev = 0;
@@ -686,20 +739,19 @@ int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename St
     if ((reinterpret_cast<uintptr_t>(x) & (sizeof(T) - 1)) || !p->standard_model()) return AS_OK;
     if (p->host.m > CPT * BT || p->host.n > BT) return AS_OK;
     const auto& q = p->packed(layout);
-    int dev = 0, sms = 0, optin = 0, occ = 0;
+    int dev = 0, occ = 0;
+    DeviceLimits D;
     AS_CUDA(cudaGetDevice(&dev));
-    AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t smem = rhs2_smem_bytes(q.n, q.m, q.nslots);
-    if (!q.compact || smem + 1024 > (size_t)optin) return AS_OK;
-    int r = ensure_uploaded(p, layout);
+    int r = device_limits(dev, &D);
     if (r) return r;
+    const size_t smem = rhs2_smem_bytes(q.n, q.m, q.nslots);
+    if (!q.compact || smem + 1024 > (size_t)D.smem_optin) return AS_OK;
+    if ((r = ensure_uploaded(p, layout))) return r;
     auto fn = &rhs_staged_kernel<V, LOGA, KMAX, EXACT, BT, CPT>;
-    AS_CUDA(raise_smem_limit((const void*)fn, smem));
-    AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, BT, smem));
+    if ((r = prepare_kernel(p, (const void*)fn, BT, smem, dev, &occ))) return r;
     if (occ < 1) return AS_OK;
     const int passes = (ns + Staged<V>::kRows - 1) / Staged<V>::kRows;
-    const int grid = std::max(1, std::min(passes, sms * occ));
+    const int grid = std::max(1, std::min(passes, D.sms * occ));
     // bulk stores need dxdt congruent with x mod 16 bytes (same staging offsets)
     const int bulk_out = ((reinterpret_cast<uintptr_t>(x) - reinterpret_cast<uintptr_t>(d)) & 15u) == 0;
     if (p->rhs_status_dev != dev) {
@@ -759,17 +811,17 @@ int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
         if (r || done) return r;
     }
     const auto& q = p->packed(prec);
-    int dev = 0, sms = 0, optin = 0, occ = 0;
+    int dev = 0, occ = 0;
+    DeviceLimits D;
     AS_CUDA(cudaGetDevice(&dev));
-    AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    AS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    int r = device_limits(dev, &D);
+    if (r || (r = ensure_uploaded(p, prec))) return r;
     const size_t vals = rhs_smem_values(q.n, q.m, q.nslots), smem = vals * sizeof(T);
     const long long stride = (long long)q.n + q.m;
-    if (q.compact && smem + 1024 <= (size_t)optin) {  // one state per CTA pass, in shared memory
+    if (q.compact && smem + 1024 <= (size_t)D.smem_optin) {  // one state per CTA pass, in shared memory
         auto fs = &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, false>;
-        AS_CUDA(raise_smem_limit((const void*)fs, smem));
-        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fs, BT, smem));
-        const int grid = std::max(1, std::min(ns, sms * std::max(occ, 1)));
+        if ((r = prepare_kernel(p, (const void*)fs, BT, smem, dev, &occ))) return r;
+        const int grid = std::max(1, std::min(ns, D.sms * std::max(occ, 1)));
         fs<<<grid, BT, smem, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, (T*)nullptr, 0ll);
     } else if (p->standard_model()) {
         // Lanes per row: a 32-byte sector once there are states for most of it.
@@ -779,8 +831,8 @@ int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
         return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 2>(p, prec, x, d, ns, st);
     } else {  // tanh variant or bias term: one CTA per state, its vectors in a global slab
         auto fg = &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, true>;
-        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fg, BT, 0));
-        const int grid = std::max(1, std::min(ns, sms * std::max(occ, 1)));
+        if ((r = prepare_kernel(p, (const void*)fg, BT, 0, dev, &occ))) return r;
+        const int grid = std::max(1, std::min(ns, D.sms * std::max(occ, 1)));
         const long long slab_stride = (long long)((vals + 63) / 64 * 64);
         AS_CUDA(p->slab[prec].alloc((size_t)grid * slab_stride * sizeof(T)));
         fg<<<grid, BT, 0, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, p->slab[prec].template as<T>(),
@@ -794,11 +846,9 @@ template <typename T, bool LOGA>
 int dispatch_rhs(as_problem* p, const T* x, T* d, int ns, void* stream) {
     if (!p || !x || !d || ns < 0) return fail(AS_ERR_BAD_INPUT, "as_rhs: null argument");
     if (ns == 0) return AS_OK;
-    constexpr int prec = sizeof(T) == 8 ? AS_PREC_F64 : AS_PREC_F32_LOGA;
-    int r = ensure_uploaded(p, prec);
-    if (r) return r;
+    if (p->host.m == 0 || p->host.k == 0) return fail(AS_ERR_NO_PROBLEM, "SAT problem has not been set");
     cudaStream_t st = (cudaStream_t)stream;
-    const int k = p->packed(prec).k;
+    const int k = p->host.k;
     if (k == 3) return launch_rhs<T, LOGA, 3, true>(p, x, d, ns, st);
     if (k == 4) return launch_rhs<T, LOGA, 4, true>(p, x, d, ns, st);
     if (k <= 16) return launch_rhs<T, LOGA, 16, false>(p, x, d, ns, st);
@@ -811,9 +861,12 @@ int launch_viol(as_problem* p, const T* x, int* c, int ns, cudaStream_t st) {
     const DevInstance& I = p->dev[prec].host_inst[0];
     const bool compact = I.lit != nullptr;
     const long long stride = (long long)I.n + I.m;
-    int dev = 0, sms = 0;
+    int dev = 0;
+    DeviceLimits D;
     AS_CUDA(cudaGetDevice(&dev));
-    AS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int r = device_limits(dev, &D);
+    if (r) return r;
+    const int sms = D.sms;
     if (compact) {  // N < 32768: the masks fit one SM
         const size_t smem = 4 * ((size_t)I.n + 1);
         // States per group: as many as 32 while every SM still gets about four CTAs (so
@@ -824,7 +877,8 @@ int launch_viol(as_problem* p, const T* x, int* c, int ns, cudaStream_t st) {
         const int per = std::max(1, std::min(32, (ns + sms * resident - 1) / (sms * resident)));
         const int grid = (ns + per - 1) / per;
         auto fn = grid > sms ? &viol_group_kernel<T, KMAX, EXACT, 256> : &viol_group_kernel<T, KMAX, EXACT, 1024>;
-        if (smem > 47 * 1024) AS_CUDA(raise_smem_limit((const void*)fn, smem));
+        int occ = 0;
+        if (smem > 47 * 1024 && (r = prepare_kernel(p, (const void*)fn, grid > sms ? 256 : 1024, smem, dev, &occ))) return r;
         fn<<<grid, grid > sms ? 256 : 1024, smem, st>>>(I, x, c, ns, stride, per);
     } else {
         const int groups = (ns + 31) / 32, gy = std::min(groups, 65535);
@@ -847,7 +901,7 @@ int dispatch_viol(as_problem* p, const T* x, int* c, int ns, void* stream) {
     int r = ensure_uploaded(p, prec);
     if (r) return r;
     cudaStream_t st = (cudaStream_t)stream;
-    const int k = p->packed(prec).k;
+    const int k = p->host.k;
     if (k == 3) return launch_viol<T, 3, true>(p, x, c, ns, st);
     if (k == 4) return launch_viol<T, 4, true>(p, x, c, ns, st);
     if (k <= 16) return launch_viol<T, 16, false>(p, x, c, ns, st);
@@ -2233,27 +2287,36 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     }
     int r = launch(av->bwd, bvals);
     if (r) return r;
-    AS_CUDA(cudaMemcpyAsync(loss, A.loss.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
-    AS_CUDA(cudaMemcpyAsync(grad_w, A.gw.p, sizeof(double) * wtot, cudaMemcpyDeviceToHost, st));
-    std::vector<float> tmp;
-    if (vb == 8) {
-        AS_CUDA(cudaMemcpyAsync(grad_x0, A.gx.p, 8 * (size_t)s->total_values, cudaMemcpyDeviceToHost, st));
-    } else {
-        tmp.resize((size_t)s->total_values);
-        AS_CUDA(cudaMemcpyAsync(tmp.data(), A.gx.p, 4 * tmp.size(), cudaMemcpyDeviceToHost, st));
-    }
-    // the recorded steps: the columns in use, gathered on the device
+    // The recorded steps: the columns in use, gathered on the device.  FP32 gradients go
+    // through pinned memory (16M values at most at a time), so that they arrive while the
+    // host still takes in the rest.
     std::vector<double> hs;
     const int used_steps = *std::max_element(ns.begin(), ns.end());
+    const size_t row = sizeof(double) * used_steps;
     if (step_sizes && used_steps > 0) {
-        const size_t row = sizeof(double) * used_steps;
         AS_CUDA(A.hsc.alloc(row * nt));
         AS_CUDA(cudaMemcpy2DAsync(A.hsc.p, row, A.hs.p, sizeof(double) * max_steps, row, nt, cudaMemcpyDeviceToDevice, st));
         hs.resize((size_t)nt * used_steps);
-        AS_CUDA(cudaMemcpyAsync(hs.data(), A.hsc.p, row * nt, cudaMemcpyDeviceToHost, st));
     }
+    const size_t gxn = (size_t)s->total_values, chunk = std::min<size_t>(gxn, 1u << 24);
+    if (vb == 4) {
+        AS_CUDA(A.pin(chunk));
+        AS_CUDA(cudaMemcpyAsync(A.pinned, A.gx.p, 4 * chunk, cudaMemcpyDeviceToHost, st));
+    } else {
+        AS_CUDA(cudaMemcpyAsync(grad_x0, A.gx.p, 8 * gxn, cudaMemcpyDeviceToHost, st));
+    }
+    AS_CUDA(cudaMemcpyAsync(loss, A.loss.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
+    AS_CUDA(cudaMemcpyAsync(grad_w, A.gw.p, sizeof(double) * wtot, cudaMemcpyDeviceToHost, st));
+    if (!hs.empty()) AS_CUDA(cudaMemcpyAsync(hs.data(), A.hsc.p, row * nt, cudaMemcpyDeviceToHost, st));
     AS_CUDA(cudaStreamSynchronize(st));
-    for (size_t i = 0; i < tmp.size(); i++) grad_x0[i] = tmp[i];
+    for (size_t o = 0; vb == 4 && o < gxn; o += chunk) {
+        const size_t c = std::min(chunk, gxn - o);
+        if (o > 0) {
+            AS_CUDA(cudaMemcpyAsync(A.pinned, A.gx.as<float>() + o, 4 * c, cudaMemcpyDeviceToHost, st));
+            AS_CUDA(cudaStreamSynchronize(st));
+        }
+        for (size_t i = 0; i < c; i++) grad_x0[o + i] = A.pinned[i];
+    }
     if (nsteps) std::copy(ns.begin(), ns.end(), nsteps);
     if (!hs.empty())
         for (int t = 0; t < nt; t++)
