@@ -436,7 +436,7 @@ struct StreamPlan {
     std::vector<int> gprob;     // problem of each group
     std::vector<size_t> goff;   // byte offset of each group's vectors in vec
     std::vector<size_t> gcand;  // word offset of each group's candidate assignments
-    DevBuf vec, lanes, tickets, active, cand;
+    DevBuf vec, stage, lanes, tickets, active, cand;
     std::vector<std::unique_ptr<DevBuf>> vstart, vpos;  // per problem occurrence lists
     std::vector<int> have_lists, nparts;                // per problem clause parts
     cudaGraphExec_t graph = nullptr;
@@ -1352,8 +1352,12 @@ size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 
 size_t stream_group_bytes(const PackedProblem& q, size_t vbytes) {
     const long long E = (long long)q.n + q.m;
-    return 6 * round256((size_t)E * kLanes * vbytes) + round256((size_t)(q.n + 1) * kLanes * vbytes) +
-           round256((size_t)q.k * q.mp * kLanes * vbytes) + round256((size_t)q.n * kLanes * vbytes);
+    return 6 * round256((size_t)E * kLanes * vbytes) + round256((size_t)(q.n + 1) * kLanes * vbytes);
+}
+// Contributions and partial sums of one stage: the groups run one after another, so they
+// share one buffer.
+size_t stream_stage_bytes(const PackedProblem& q, size_t vbytes) {
+    return round256((size_t)q.k * q.mp * kLanes * vbytes) + round256((size_t)q.n * kLanes * vbytes);
 }
 
 template <typename T>
@@ -1372,12 +1376,12 @@ StreamArgs<T> stream_args(as_solver* s, int g, const unsigned long long* deadlin
     A.K4 = reinterpret_cast<T*>(base + 4 * vb);
     A.K5 = reinterpret_cast<T*>(base + 5 * vb);
     A.SY = reinterpret_cast<T*>(base + 6 * vb);
-    A.CS = reinterpret_cast<T*>(base + 6 * vb + round256((size_t)(q.n + 1) * kLanes * sizeof(T)));
+    A.CS = P.stage.as<T>();
     A.lanes = P.lanes.as<LaneState>() + (size_t)g * kLanes;
     A.vstart = P.vstart[p]->as<int>();
     A.vpos = P.vpos[p]->as<int>();
-    A.ACC = reinterpret_cast<T*>(base + 6 * vb + round256((size_t)(q.n + 1) * kLanes * sizeof(T)) +
-                                 round256((size_t)q.k * q.mp * kLanes * sizeof(T)));
+    const size_t cs_bytes = round256((size_t)q.k * q.mp * kLanes * sizeof(T));
+    A.ACC = reinterpret_cast<T*>(static_cast<char*>(P.stage.p) + cs_bytes);
     A.m0 = 0;
     A.m1 = q.m;
     A.part = 0;
@@ -1468,7 +1472,7 @@ int stream_plan(as_solver* s) {
     P.gcand.clear();
     std::vector<LaneState> lanes;
     const size_t vbytes = s->precision == AS_PREC_F64 ? 8 : 4;
-    size_t total = 0, cand_words = 0;
+    size_t total = 0, stage = 0, cand_words = 0;
     for (int u = 0; u < num_traj;) {
         const int p = pi[s->order[u]];
         const auto& q = s->problems[p];
@@ -1476,6 +1480,7 @@ int stream_plan(as_solver* s) {
         P.goff.push_back(total);
         P.gcand.push_back(cand_words);
         total += stream_group_bytes(q, vbytes);
+        stage = std::max(stage, stream_stage_bytes(q, vbytes));
         cand_words += (size_t)kLanes * ((q.n + 31) / 32);
         for (int l = 0; l < kLanes; l++) {
             LaneState L;
@@ -1512,6 +1517,7 @@ int stream_plan(as_solver* s) {
             if (r) return r;
         }
     AS_CUDA(P.vec.alloc(std::max<size_t>(total, 256)));
+    AS_CUDA(P.stage.alloc(std::max<size_t>(stage, 256)));
     AS_CUDA(P.lanes.alloc(sizeof(LaneState) * lanes.size()));
     AS_CUDA(P.tickets.alloc(sizeof(int) * 2 * P.ngroups));
     AS_CUDA(P.active.alloc(sizeof(int) * P.ngroups));
@@ -1533,6 +1539,22 @@ int stream_plan(as_solver* s) {
     AS_CUDA(cudaMemcpy(s->unit_state.p, us.data(), sizeof(long long) * num_traj, cudaMemcpyHostToDevice));
     AS_CUDA(cudaMemcpy(s->unit_bits.p, ub.data(), sizeof(long long) * num_traj, cudaMemcpyHostToDevice));
     return AS_OK;
+}
+
+// The clause and variable kernels of stage S: compiled for the stage where the clause
+// length is exact (fewer registers for early stages, no runtime choice per element).
+template <typename T, bool LOGA, int KMAX, bool EXACT>
+std::pair<void (*)(StreamArgs<T>), void (*)(StreamArgs<T>)> stream_stage_fn(int S) {
+#define AS_STAGE(N) {&stream_clause_kernel<T, LOGA, KMAX, EXACT, EXACT ? N : 0>, &stream_var_kernel<T, LOGA, N>}
+    switch (S) {
+        case 1: return AS_STAGE(1);
+        case 2: return AS_STAGE(2);
+        case 3: return AS_STAGE(3);
+        case 4: return AS_STAGE(4);
+        case 5: return AS_STAGE(5);
+        default: return AS_STAGE(6);
+    }
+#undef AS_STAGE
 }
 
 // One pass (an RK attempt of every lane) of every group, in stream order.
@@ -1557,8 +1579,8 @@ int stream_record_pass(as_solver* s, cudaStream_t st, const unsigned long long* 
                 A.vstart = vstart0 + (size_t)part * n;
                 const int gcp = (int)std::max(1ll, std::min(((long long)kRowThreads * (A.m1 - A.m0) + BT - 1) / BT,
                                                             (long long)sms * 8));
-                stream_clause_kernel<T, LOGA, KMAX, EXACT><<<gcp, BT, 0, st>>>(A);
-                stream_var_kernel<T, LOGA><<<gv, BT, 0, st>>>(A);
+                stream_stage_fn<T, LOGA, KMAX, EXACT>(S).first<<<gcp, BT, 0, st>>>(A);
+                stream_stage_fn<T, LOGA, KMAX, EXACT>(S).second<<<gv, BT, 0, st>>>(A);
             }
         }
         A.vstart = vstart0;
@@ -1622,7 +1644,7 @@ int stream_run(as_solver* s) {
         bool any = false;
         for (int a : act) any |= a != 0;
         if (!any) break;
-        chunk = std::min(chunk * 2, 16);
+        chunk = std::min(chunk * 2, 8);  // passes behind the last one return at once, but cost launches
     }
     for (int g = 0; g < P.ngroups; g++) {
         StreamArgs<T> A = stream_args<T>(s, g, deadline);

@@ -140,6 +140,14 @@ template <> struct Lit<1> {
     __device__ __forceinline__ bool neg() const { return (w >> 31) != 0; }
 };
 
+// A literal's variable and sign alone (no contribution slot).
+template <int ENC> struct Var {
+    uint32_t w;
+    __device__ __forceinline__ void load(const DevInstance& I, int idx) { w = ld_ro((ENC ? I.litw : I.lit) + idx); }
+    __device__ __forceinline__ uint32_t var() const { return ENC ? w & 0x7fffffffu : (w >> 16) & 0x7fffu; }
+    __device__ __forceinline__ bool neg() const { return (w >> 31) != 0; }
+};
+
 // Clause phase for one clause m: stores the per-literal spin contributions into cs
 // and returns da_m (du_m in log space).  `am` is a_m in linear space.
 // EXACT: every clause has exactly KMAX slots (shorter clauses are padded with the
@@ -277,7 +285,7 @@ __device__ __forceinline__ int clause_violated(const DevInstance& I, int m, cons
 #pragma unroll
     for (int q = 0; q < KMAX; q++) {
         if (EXACT || q < I.k) {
-            Lit<ENC> w;
+            Var<ENC> w;
             w.load(I, q * I.mp + m);
             const bool t = sy[w.var()] > T(0);
             sat |= w.neg() ? !t : t;

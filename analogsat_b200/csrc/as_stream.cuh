@@ -35,6 +35,14 @@
 //    kernel (ticket counter, no waiting); the post kernel commits accepted states,
 //    counts unsat clauses for lanes at a batch end and applies SatSolver's status
 //    rules in its last block.  No kernel waits on another block.
+// The stage kernels are compiled per stage (STAGE; 0: the stage of the arguments, for
+// clause lengths up to 16): with the stage at run time every thread held all six stage
+// vectors of a row and chose among six input formulas per lane, 80 registers and a third of
+// the warps.  N = 1e5, M = 1e6, K = 4, a group of eight lanes: clause kernels 59-76 us, variable
+// kernels 54-58 us a launch so; a pass of four groups 2.95 ms, 2.4 ms now (48 and 32 registers
+// but for stage 6, and one word per literal read instead of two), about 5 TB/s of DRAM
+// traffic.  L2 eviction hints (contributions kept, stage vectors leaving first) measured 0 to
+// 12% slower: half of L2 is nearer to each SM, and the 128 MB of contributions fit neither half.
 // Per-lane arithmetic mirrors clause_phase / var_phase / stage_in / rk_new /
 // rk_err_ratio and the controller of solve_kernel operation for operation; with the
 // explicitly rounded FP64 arithmetic a lane follows solve_kernel's trajectory bit for
@@ -192,13 +200,13 @@ __device__ __forceinline__ T* stage_out(const StreamArgs<T>& A, int S) {
 // products (clause_phase's expression order, per lane), contributions into CS,
 // da_m -> K_S (stage 6: xnew -> K2 and the error ratio).  kRowThreads threads per
 // clause, kSub lanes each.
-template <typename T, bool LOGA, int KMAX, bool EXACT>
+template <typename T, bool LOGA, int KMAX, bool EXACT, int STAGE>
 __global__ void __launch_bounds__(256) stream_clause_kernel(StreamArgs<T> A) {
     using Ar = Arith<T>;
     __shared__ double red[kLanes * 32];
     if (*A.active == 0) return;
     const DevInstance& I = A.I;
-    const int S = A.S, n = I.n;
+    const int S = STAGE ? STAGE : A.S, n = I.n;
     const int lb = (threadIdx.x % kRowThreads) * kSub;  // first lane of this thread
     T h[kSub], h0[kSub];
     load_lane_steps(A.lanes + lb, h, h0);
@@ -219,7 +227,7 @@ __global__ void __launch_bounds__(256) stream_clause_kernel(StreamArgs<T> A) {
             if constexpr (LOGA) am.v[l] = exp2_fast(y.v[l]);
             else am.v[l] = y.v[l];
         }
-        Lit<1> w[KMAX];
+        Var<1> w[KMAX];
         T f[KMAX][kSub];
         T km[kSub];
 #pragma unroll
@@ -350,14 +358,14 @@ __device__ __forceinline__ void lane_decide(LaneState& L, const StreamArgs<T>& A
 // Stage S, variable side: occurrence-list sums -> K_S and the spin input of stage
 // S + 1 (stage 6: xnew -> K2, the error ratio, and in the last block the lanes'
 // decisions).  kRowThreads threads per variable, kSub lanes each.
-template <typename T, bool LOGA>
+template <typename T, bool LOGA, int STAGE>
 __global__ void __launch_bounds__(256) stream_var_kernel(StreamArgs<T> A) {
     using Ar = Arith<T>;
     __shared__ double red[kLanes * 32];
     __shared__ int s_flag;
     if (*A.active == 0) return;
     const DevInstance& I = A.I;
-    const int S = A.S, n = I.n;
+    const int S = STAGE ? STAGE : A.S, n = I.n;
     const int lb = (threadIdx.x % kRowThreads) * kSub;
     T h[kSub], h0[kSub];
     load_lane_steps(A.lanes + lb, h, h0);
@@ -473,7 +481,7 @@ __global__ void __launch_bounds__(256) stream_post_kernel(StreamArgs<T> A, int n
 #pragma unroll
                 for (int q = 0; q < KMAX; q++) {
                     if (EXACT || q < I.k) {
-                        Lit<1> w;
+                        Var<1> w;
                         w.load(I, q * I.mp + m);
                         const bool real = w.var() < (uint32_t)n;
 #pragma unroll
