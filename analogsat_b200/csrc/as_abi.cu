@@ -75,7 +75,7 @@ struct DevBuf {
 // Device copy of one or more packed instances in a single pool.
 struct DevicePool {
     int device = -1;
-    DevBuf lit, litw, slotw, srow, perm, iperm, icperm, cperm, deg, inst, flit;
+    DevBuf lit, litw, slotw, srow, perm, iperm, icperm, cperm, inst, flit;
     DevBuf plit, pc0, psrow, pcnt, picperm;  // clause-parts layouts (lean global-rows form)
     std::vector<DevInstance> host_inst;
 
@@ -101,9 +101,8 @@ struct DevicePool {
         AS_CUDA(litw.alloc(std::max<size_t>(nw, 1) * 4));
         AS_CUDA(slotw.alloc(std::max<size_t>(nw, 1) * 4));
         AS_CUDA(srow.alloc(std::max<size_t>(nr, 1) * 4));
-        AS_CUDA(perm.alloc(std::max<size_t>(np, 1) * 4));
+        AS_CUDA(perm.alloc(std::max<size_t>(np, 1) * 8));  // the degrees behind the permutations
         AS_CUDA(iperm.alloc(std::max<size_t>(np, 1) * 4));
-        AS_CUDA(deg.alloc(std::max<size_t>(np, 1) * 4));
         AS_CUDA(icperm.alloc(std::max<size_t>(nc, 1) * 4));
         AS_CUDA(cperm.alloc(std::max<size_t>(nc, 1) * 4));
         AS_CUDA(inst.alloc(sizeof(DevInstance) * std::max<size_t>(pk.size(), 1)));
@@ -179,7 +178,7 @@ struct DevicePool {
             d.srow = srow.as<int32_t>() + orr;
             d.perm = perm.as<int32_t>() + op;
             d.iperm = iperm.as<int32_t>() + op;
-            d.deg = deg.as<int32_t>() + op;
+            d.deg = perm.as<int32_t>() + np + op;
             d.icperm = icperm.as<int32_t>() + oc;
             d.cperm = cperm.as<int32_t>() + oc;
             {
@@ -201,7 +200,7 @@ struct DevicePool {
             int r;
             if ((r = put(lit, ol, q->lit)) || (r = put(litw, ow, q->litw)) || (r = put(slotw, ow, q->slotw)) ||
                 (r = put(srow, orr, q->srow)) || (r = put(perm, op, q->perm)) ||
-                (r = put(iperm, op, q->iperm)) || (r = put(deg, op, q->deg)) || (r = put(icperm, oc, q->icperm)) ||
+                (r = put(iperm, op, q->iperm)) || (r = put(perm, np + op, q->deg)) || (r = put(icperm, oc, q->icperm)) ||
                 (r = put(cperm, oc, q->cperm)))
                 return r;
             ol += q->lit.size();
@@ -503,7 +502,7 @@ struct as_solver {
     long long total_values = 0;
     std::vector<int> order;            // launch order -> user trajectory
     struct Group {
-        int variant, u0, u1, bt, occ, ctas;
+        int variant, u0, u1, bt, occ, ctas, mmax;
         size_t smem, slab_off;
         long long slab_stride;
     };
@@ -512,6 +511,9 @@ struct as_solver {
     DevBuf states, results, unit_inst, unit_state, unit_bits, queue, solved, deadline, best_bits, slab;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;  // orders a caller's stream with `stream`
+    std::vector<cudaStream_t> side;                 // launch groups after the first run beside it
+    std::vector<cudaEvent_t> side_done;
+    cudaEvent_t ev_fork = nullptr;
     cudaGraphExec_t graph = nullptr;
     bool graph_valid = false;
     bool groups_dirty = true;
@@ -522,6 +524,9 @@ struct as_solver {
         if (graph) cudaGraphExecDestroy(graph);
         if (ev_in) cudaEventDestroy(ev_in);
         if (ev_out) cudaEventDestroy(ev_out);
+        if (ev_fork) cudaEventDestroy(ev_fork);
+        for (cudaEvent_t e : side_done) cudaEventDestroy(e);
+        for (cudaStream_t t : side) cudaStreamDestroy(t);
         if (stream) cudaStreamDestroy(stream);
     }
     void invalidate() { graph_valid = false; }
@@ -1046,7 +1051,7 @@ int32_t as_solver_set_wall_budget(as_solver* s, double v) {
 }
 int32_t as_solver_set_stop_on_first(as_solver* s, int32_t f) {
     if (!s) return fail(AS_ERR_BAD_INPUT, "null solver");
-    s->stop_on_first = f ? 1 : 0; s->invalidate();
+    s->stop_on_first = f ? 1 : 0; s->groups_dirty = true; s->invalidate();
     return AS_OK;
 }
 int32_t as_solver_set_track_best(as_solver* s, int32_t f) {
@@ -1117,11 +1122,18 @@ int build_groups(as_solver* s) {
             return fail(AS_ERR_UNSUPPORTED, "no compiled launch shape fits problem " + std::to_string(p));
     }
     // global-storage problems with few trajectories: spread each trajectory over a
-    // cluster of CTAs so that all trajectories run at once on the whole GPU
+    // cluster of CTAs so that all trajectories run at once on the whole GPU.  Not those of the
+    // lean kernel in one clause part: its gathers on chip make one CTA faster than a cluster
+    // of four or eight with everything in L2 (us per RHS, one CTA / automatic cluster: N = 1500,
+    // 1 start 4.3 / 8.1, 16 starts 4.3 / 14.7; N = 3000 7.8 / 10.8 and 7.9 / 19.0), with the same
+    // operations.  In two parts (N = 4900) 17.6 / 14.0 with 8 starts, 17.0 / 21.2 with 30.
     {
         std::vector<int> per_problem(np, 0);
         for (int t = 0; t < num_traj; t++) per_problem[s->traj_problem[t]]++;
         long gs_units = 0;
+        auto clustered = [&](int p) {
+            return vs[pv[p]].gs && !(vs[pv[p]].lean && s->problems[p].lean_parts == 1 && !s->forced_cl);
+        };
         for (int p = 0; p < np; p++)
             if (vs[pv[p]].gs) gs_units += per_problem[p];
         bool bias = false;  // the bias term's clause-weight sum is reduced per CTA
@@ -1136,7 +1148,7 @@ int build_groups(as_solver* s) {
         if (want_cl > 1 && !s->forced_bt) {
             for (int p = 0; p < np; p++) {
                 const Variant& cur = vs[pv[p]];
-                if (!cur.gs) continue;
+                if (!clustered(p)) continue;
                 for (int i = 0; i < (int)vs.size(); i++)
                     if (vs[i].gs && vs[i].cl == want_cl && vs[i].precision == cur.precision &&
                         vs[i].kmax == cur.kmax && vs[i].exact == cur.exact)
@@ -1145,11 +1157,14 @@ int build_groups(as_solver* s) {
         }
     }
     const auto& pi = s->traj_problem;
-    // Within a launch shape the work queue deals the problems round-robin (the r-th
-    // trajectory of every problem before the (r+1)-th of any), so the trajectories
-    // running at once belong to different problems: with stop-on-first an instance's
-    // restarts then run a few at a time instead of filling the GPU together and being
-    // stopped together.
+    // With stop-on-first the work queue of a launch shape deals the problems round-robin
+    // (the r-th trajectory of every problem before the (r+1)-th of any), so the trajectories
+    // running at once belong to different problems: an instance's restarts then run a few
+    // at a time instead of filling the GPU together and being stopped together.  Otherwise
+    // every trajectory runs to its own end, and the largest instances go first: a long
+    // trajectory that starts last leaves the other SMs idle (264 trajectories of N = 100 to
+    // 5000, 100 steps: 17.2 ms dealt round-robin, 14.1 so).
+    const bool largest_first = !s->stop_on_first;
     std::vector<int> rank(num_traj), seen(np, 0);
     for (int t = 0; t < num_traj; t++) rank[t] = seen[pi[t]]++;
     s->order.resize(num_traj);
@@ -1157,6 +1172,8 @@ int build_groups(as_solver* s) {
     std::stable_sort(s->order.begin(), s->order.end(), [&](int a, int b) {
         const int va = pv[pi[a]], vb = pv[pi[b]];
         if (va != vb) return va < vb;
+        const int ma = s->problems[pi[a]].m, mb = s->problems[pi[b]].m;
+        if (largest_first && ma != mb) return ma > mb;
         if (rank[a] != rank[b]) return rank[a] < rank[b];
         return pi[a] < pi[b];
     });
@@ -1179,6 +1196,7 @@ int build_groups(as_solver* s) {
         G.variant = vi;
         G.u0 = u;
         G.u1 = e;
+        G.mmax = mmax;
         // global storage: 512 threads (two CTAs per SM) while the in-flight slabs fit in
         // L2, else 1,024 (one per SM, half the slabs)
         int gs_bt = 512;
@@ -1229,6 +1247,15 @@ int build_groups(as_solver* s) {
         u = e;
     }
     if (slab_total) AS_CUDA(s->slab.alloc(slab_total));
+    if (s->groups.size() > 1 && !s->ev_fork) AS_CUDA(cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming));
+    while (s->side_done.size() + 1 < s->groups.size()) {  // streams of the groups beside the first (record_solve)
+        cudaStream_t t;
+        cudaEvent_t e;
+        AS_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+        s->side.push_back(t);
+        AS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        s->side_done.push_back(e);
+    }
     std::vector<int> ui(num_traj);
     std::vector<long long> us(num_traj), ub(num_traj);
     for (int u = 0; u < num_traj; u++) {
@@ -1283,10 +1310,27 @@ int record_solve(as_solver* s, cudaStream_t st) {
                                                (unsigned long long)(s->wall_budget * 1e9));
         AS_CUDA(cudaGetLastError());
     }
-    for (size_t g = 0; g < s->groups.size(); g++) {
+    // The groups, those of the largest instances first, each but the first on a stream of
+    // its own between a fork and a join: the CTAs of a later group start where an earlier one
+    // leaves SMs free, from the start or in its tail (264 trajectories of N = 100 to 5000, 100
+    // steps: 14.1 ms one after another, 12.4 so; 512 instances x 64 starts with stop-on-first:
+    // 1,840 instances/s, 1,936 so).
+    std::vector<size_t> by_size(s->groups.size());
+    for (size_t g = 0; g < by_size.size(); g++) by_size[g] = g;
+    std::stable_sort(by_size.begin(), by_size.end(),
+                     [&](size_t a, size_t b) { return s->groups[a].mmax > s->groups[b].mmax; });
+    const bool fork = s->groups.size() > 1;
+    if (fork) AS_CUDA(cudaEventRecord(s->ev_fork, st));
+    const cudaStream_t main_stream = st;
+    for (size_t i = 0; i < by_size.size(); i++) {
+        const size_t g = by_size[i];
         const auto& G = s->groups[g];
         const Variant& v = vs[G.variant];
         const size_t smem = G.smem;
+        if (fork && i > 0) {
+            st = s->side[i - 1];
+            AS_CUDA(cudaStreamWaitEvent(st, s->ev_fork, 0));
+        }
         const int occ = G.occ, ctas = G.ctas, units = G.u1 - G.u0;
         SolveParams P;
         P.inst = s->pool.inst.as<DevInstance>();
@@ -1325,8 +1369,14 @@ int record_solve(as_solver* s, cudaStream_t st) {
         } else {
             AS_CUDA(cudaLaunchKernel((const void*)v.fn, dim3(ctas), dim3(G.bt), args, smem, st));
         }
-        s->last_bt = G.bt; s->last_ctas = ctas; s->last_smem = (int)smem; s->last_occ = occ;
-        s->last_kernel = v.name();
+        if (fork && i > 0) {
+            AS_CUDA(cudaEventRecord(s->side_done[i - 1], st));
+            AS_CUDA(cudaStreamWaitEvent(main_stream, s->side_done[i - 1], 0));
+        }
+        if (g + 1 == s->groups.size()) {
+            s->last_bt = G.bt; s->last_ctas = ctas; s->last_smem = (int)smem; s->last_occ = occ;
+            s->last_kernel = v.name();
+        }
     }
     return AS_OK;
 }
