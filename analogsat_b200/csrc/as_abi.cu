@@ -735,22 +735,32 @@ template <typename V, bool LOGA, int KMAX, bool EXACT, int BT>
 int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename Staged<V>::T* d, int ns,
                       cudaStream_t st, bool* done) {
     using T = typename Staged<V>::T;
-    constexpr int CPT = 5;  // instances whose footprint fits have M <= 5 * 1024
-    constexpr int layout = sizeof(T) == 8 ? AS_PREC_F64 : kLayoutPair;
+    constexpr bool one = sizeof(V) == 4;  // one FP32 state per pass
+    constexpr int CPT = one ? 6 : 5;      // pairs that fit have M <= 5 * 1024
+    constexpr int layout = sizeof(T) == 8 ? AS_PREC_F64 : one ? AS_PREC_F32_LOGA : kLayoutPair;
     *done = false;
-    if constexpr (BT < 1024)
-        if (p->host.n > BT || p->host.m > CPT * BT)
-            return launch_rhs_staged<V, LOGA, KMAX, EXACT, 2 * BT>(p, x, d, ns, st, done);
     if ((reinterpret_cast<uintptr_t>(x) & (sizeof(T) - 1)) || !p->standard_model()) return AS_OK;
-    if (p->host.m > CPT * BT || p->host.n > BT) return AS_OK;
+    if constexpr (!one) {
+        if (p->host.n > BT || p->host.m > CPT * BT) {
+            if constexpr (BT < 1024) return launch_rhs_staged<V, LOGA, KMAX, EXACT, 2 * BT>(p, x, d, ns, st, done);
+            else if constexpr (sizeof(T) == 4)
+                return launch_rhs_staged<float, LOGA, KMAX, EXACT, BT>(p, x, d, ns, st, done);
+            else return AS_OK;
+        }
+    }
+    if (p->host.n >= 32768) return AS_OK;  // never compact
     const auto& q = p->packed(layout);
     int dev = 0, occ = 0;
     DeviceLimits D;
     AS_CUDA(cudaGetDevice(&dev));
     int r = device_limits(dev, &D);
     if (r) return r;
-    const size_t smem = rhs2_smem_bytes(q.n, q.m, q.nslots);
-    if (!q.compact || smem + 1024 > (size_t)D.smem_optin) return AS_OK;
+    const size_t smem = one ? rhs1_smem_bytes(q.n, q.m, q.nslots) : rhs2_smem_bytes(q.n, q.m, q.nslots);
+    if (!q.compact || smem + 1024 > (size_t)D.smem_optin) {
+        if constexpr (sizeof(V) == 8 && sizeof(T) == 4 && BT == 1024)  // pairs that do not fit
+            return launch_rhs_staged<float, LOGA, KMAX, EXACT, BT>(p, x, d, ns, st, done);
+        return AS_OK;
+    }
     if ((r = ensure_uploaded(p, layout))) return r;
     auto fn = &rhs_staged_kernel<V, LOGA, KMAX, EXACT, BT, CPT>;
     if ((r = prepare_kernel(p, (const void*)fn, BT, smem, dev, &occ))) return r;

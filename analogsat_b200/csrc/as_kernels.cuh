@@ -520,11 +520,12 @@ __global__ void __launch_bounds__(BT) rhs_batch_kernel(DevInstance I, const T* _
 }
 
 // ---------------------------------------------------------------------------
-// Standalone batched RHS with staged states: one element type V of 8 bytes per shared
-// array element -- float2: two FP32 states per CTA pass, so the literal loads, index
+// Standalone batched RHS with staged states: one value of type V per shared array
+// element -- float2: two FP32 states per CTA pass, so the literal loads, index
 // arithmetic and loop control are shared by the two and the arithmetic runs as packed
-// FP32x2 (FFMA2/FMUL2/FADD2); double: one FP64 state.  Products are formed in the one-state
-// kernel's order.
+// FP32x2 (FFMA2/FMUL2/FADD2); double: one FP64 state; float: one FP32 state, for instances
+// whose pairs do not fit (N from about 1,000 to 2,300 at alpha 4.2).  Products are formed in
+// the one-state kernel's order.
 //
 // Data movement: the public states of a pass (contiguous in HBM) arrive in a shared
 // staging buffer with one 1-D bulk copy (cp.async.bulk, mbarrier completion) that is
@@ -548,7 +549,9 @@ __global__ void __launch_bounds__(BT) rhs_batch_kernel(DevInstance I, const T* _
 // 19 / 28 / 45 / 84 us so.
 // FP64, 1,999 states of N = 777, M = 3301: 104 us with the one-state kernel (no room for a
 // second CTA on the SM, so its loads, phases and stores run one after another), 63 us here =
-// 2.1 TB/s; 16,384 states of N = 120: 122 us against 68.  Bound by shared-memory wavefronts
+// 2.1 TB/s; 16,384 states of N = 120: 122 us against 68.  One FP32 state per pass, its words
+// read again from L2: 5,906 states of N = 1400 258 us with the one-state kernel, 152 us here,
+// 4,134 of N = 2000 383 and 153 us.  Bound by shared-memory wavefronts
 // (gathers, slot stores and sums: about 4,500 per FP32 pair of N = 1000, M = 4250) and, around
 // them, by two barriers a pass.
 // ---------------------------------------------------------------------------
@@ -558,6 +561,11 @@ __host__ __device__ inline size_t rhs2_stage_floats(long long stride) {
 __host__ __device__ inline size_t rhs2_smem_bytes(int n, int m, int nslots) {
     return 16 + 8 * rhs2_stage_floats((long long)n + m) +
            8 * ((size_t)((n + 1 + 3) & ~3) + (size_t)nslots + 1);
+}
+// ... with one FP32 state per pass
+__host__ __device__ inline size_t rhs1_stage_floats(long long stride) { return (size_t)((stride + 3 + 3) & ~3ll); }
+__host__ __device__ inline size_t rhs1_smem_bytes(int n, int m, int nslots) {
+    return 16 + 8 * rhs1_stage_floats((long long)n + m) + 4 * ((size_t)((n + 1 + 3) & ~3) + (size_t)nslots + 1);
 }
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
@@ -600,6 +608,25 @@ template <> struct Staged<float2> {
     static __device__ __forceinline__ float2 contribution(float2 r, float2 prod, uint32_t w) {
         return __fmul2_rn(__fmul2_rn(r, prod), f2(__int_as_float((w & 0x80000000u) ^ 0xBF800000u)));
     }
+};
+// One FP32 state: instances too large for pairs of them.
+template <> struct Staged<float> {
+    using T = float;
+    static constexpr int kRows = 1;
+    static __device__ __forceinline__ float splat(float a) { return a; }
+    static __device__ __forceinline__ float get(const float* r0, const float*, int e) { return r0[e]; }
+    static __device__ __forceinline__ void put(float* r0, float*, int e, float v) { r0[e] = v; }
+    static __device__ __forceinline__ float add(float a, float b) { return a + b; }
+    static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
+    static __device__ __forceinline__ float flip(float a, uint32_t w) {
+        return __int_as_float(__float_as_int(a) ^ (int)(w & 0x80000000u));
+    }
+    static __device__ __forceinline__ float factor(uint32_t w, float s) { return 1.0f - flip(s, w); }
+    static __device__ __forceinline__ float product(float km, float f, bool first) { return first ? f : km * f; }
+    static __device__ __forceinline__ float weight(float P, float kn, float am) { return P * (am * (2.0f * kn * kn)); }
+    static __device__ __forceinline__ float dlog(float P, float kn) { return (P * P) * (kn * kn * kInvLn2); }
+    static __device__ __forceinline__ float da(float P, float kn, float am) { return ((am * (kn * kn)) * P) * P; }
+    static __device__ __forceinline__ float contribution(float r, float prod, uint32_t w) { return flip(r * prod, w); }
 };
 template <> struct Staged<double> {
     using T = double;
@@ -703,9 +730,49 @@ struct PassCopy {
     }
 };
 
+// Clause phase of one clause: a_m in, da_m out at the public clause position j, the
+// literals' contributions into their slots.
+template <typename V, bool LOGA, int KMAX, bool EXACT>
+__device__ __forceinline__ void staged_clause(const DevInstance& I, const Lit<0>* w, int j, const V* sy, V* cs,
+                                              typename Staged<V>::T* S0, typename Staged<V>::T* S1,
+                                              typename Staged<V>::T knorm) {
+    using O = Staged<V>;
+    using T = typename O::T;
+    V f[KMAX];
+    V km = O::splat(knorm);
+#pragma unroll
+    for (int q = 0; q < KMAX; q++) {
+        if (EXACT || q < I.k) {
+            f[q] = O::factor(w[q].w, sy[w[q].var()]);
+            km = O::product(km, f[q], q == 0);
+        }
+    }
+    V am = O::get(S0, S1, j);
+    if constexpr (LOGA && O::kRows == 2) am = make_float2(exp2_fast(am.x), exp2_fast(am.y));
+    else if constexpr (LOGA) am = exp2_fast(am);
+    if constexpr (LOGA) O::put(S0, S1, j, O::dlog(km, knorm));
+    else O::put(S0, S1, j, O::da(km, knorm, am));
+    const V r = O::weight(km, knorm, am);
+#pragma unroll
+    for (int q = 0; q < KMAX; q++) {
+        if (EXACT || q < I.k) {
+            V prod = O::splat(T(1));
+            bool first = true;
+#pragma unroll
+            for (int l = 0; l < KMAX; l++) {
+                if (l != q && (EXACT || l < I.k)) {
+                    prod = first ? f[l] : O::mul(prod, f[l]);
+                    first = false;
+                }
+            }
+            cs[w[q].slot()] = O::contribution(r, prod, w[q].w);
+        }
+    }
+}
+
 // CPT: clauses per thread (M <= CPT BT, N <= BT); a thread's literal words, public clause
 // and variable indices and SELL rows are the same for every pass, so they are loaded once
-// into registers.
+// into registers.  CPT > 5: any M and N, the records read again in each pass.
 template <typename V, bool LOGA, int KMAX, bool EXACT, int BT, int CPT>
 __global__ void __launch_bounds__(BT, 1024 / BT)
     rhs_staged_kernel(DevInstance I, const typename Staged<V>::T* __restrict__ x,
@@ -717,7 +784,8 @@ __global__ void __launch_bounds__(BT, 1024 / BT)
     using Copy = PassCopy<T, ROWS>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
-    const size_t sf = rhs2_stage_floats(stride) * 4 / sizeof(T);
+    constexpr bool REG = CPT <= 5;  // literal words and variable records in registers, else read per pass
+    const size_t sf = sizeof(V) == 4 ? rhs1_stage_floats(stride) : rhs2_stage_floats(stride) * 4 / sizeof(T);
     T* stg0 = reinterpret_cast<T*>(smem_raw + 16);
     V* sy = reinterpret_cast<V*>(stg0 + 2 * sf);
     V* cs = sy + ((I.n + 1 + 3) & ~3);
@@ -734,16 +802,18 @@ __global__ void __launch_bounds__(BT, 1024 / BT)
         mbar_init(bar, 1);
         mbar_init(bar + 1, 1);
     }
-    Lit<0> lw[CPT][KMAX];
-    int lj[CPT];
+    Lit<0> lw[REG ? CPT : 1][KMAX];
+    int lj[REG ? CPT : 1];
+    if constexpr (REG) {
 #pragma unroll
-    for (int i = 0; i < CPT; i++) {
-        const int m = tid + i * BT;
-        lj[i] = m < I.m ? n + ld_ro(I.cperm + m) : 0;
+        for (int i = 0; i < CPT; i++) {
+            const int m = tid + i * BT;
+            lj[i] = m < I.m ? n + ld_ro(I.cperm + m) : 0;
 #pragma unroll
-        for (int q = 0; q < KMAX; q++)
-            if (m < I.m && (EXACT || q < I.k)) lw[i][q].load(I, q * I.mp + m);
-            else lw[i][q].w = 0;
+            for (int q = 0; q < KMAX; q++)
+                if (m < I.m && (EXACT || q < I.k)) lw[i][q].load(I, q * I.mp + m);
+                else lw[i][q].w = 0;
+        }
     }
     const bool has_v = tid < n;  // one variable per thread
     const int vp = has_v ? __ldg(I.perm + tid) : 0;
@@ -777,6 +847,8 @@ __global__ void __launch_bounds__(BT, 1024 / BT)
         const T* A0 = stg0 + (size_t)b * sf + c.off;
         const T* A1 = ROWS == 2 && 2 * q + 1 < ntraj ? A0 + stride : A0;
         if (has_v) sy[tid] = O::get(A0, A1, vp);
+        if constexpr (!REG)
+            for (int v = tid + BT; v < n; v += BT) sy[v] = O::get(A0, A1, __ldg(I.perm + v));
     };
     uint32_t parity = 0;   // bit b: phase parity expected next on bar[b]
     uint32_t pending = 1;  // bit b: a copy into buffer b not yet waited for (same in all threads)
@@ -801,39 +873,20 @@ __global__ void __launch_bounds__(BT, 1024 / BT)
         T* S0 = stg0 + (size_t)b * sf + cur.off;
         T* S1 = two ? S0 + stride : S0;
         // clause phase: a_m in, da_m out at the public clause position
+        if constexpr (REG) {
 #pragma unroll
-        for (int i = 0; i < CPT; i++) {
-            if (tid + i * BT >= I.m) break;
-            const Lit<0>* w = lw[i];
-            V f[KMAX];
-            V km = O::splat(knorm);
-            const int j = lj[i];
-#pragma unroll
-            for (int q = 0; q < KMAX; q++) {
-                if (EXACT || q < I.k) {
-                    f[q] = O::factor(w[q].w, sy[w[q].var()]);
-                    km = O::product(km, f[q], q == 0);
-                }
+            for (int i = 0; i < CPT; i++) {
+                if (tid + i * BT >= I.m) break;
+                staged_clause<V, LOGA, KMAX, EXACT>(I, lw[i], lj[i], sy, cs, S0, S1, knorm);
             }
-            V am = O::get(S0, S1, j);
-            if constexpr (LOGA) am = make_float2(exp2_fast(am.x), exp2_fast(am.y));
-            if constexpr (LOGA) O::put(S0, S1, j, O::dlog(km, knorm));
-            else O::put(S0, S1, j, O::da(km, knorm, am));
-            const V r = O::weight(km, knorm, am);
+        } else {
+#pragma unroll 2
+            for (int m = tid; m < I.m; m += BT) {
+                Lit<0> w[KMAX];
 #pragma unroll
-            for (int q = 0; q < KMAX; q++) {
-                if (EXACT || q < I.k) {
-                    V prod = O::splat(T(1));
-                    bool first = true;
-#pragma unroll
-                    for (int l = 0; l < KMAX; l++) {
-                        if (l != q && (EXACT || l < I.k)) {
-                            prod = first ? f[l] : O::mul(prod, f[l]);
-                            first = false;
-                        }
-                    }
-                    cs[w[q].slot()] = O::contribution(r, prod, w[q].w);
-                }
+                for (int q = 0; q < KMAX; q++)
+                    if (EXACT || q < I.k) w[q].w = __ldg(I.lit + q * I.mp + m);
+                staged_clause<V, LOGA, KMAX, EXACT>(I, w, n + __ldg(I.cperm + m), sy, cs, S0, S1, knorm);
             }
         }
         __syncthreads();
@@ -852,6 +905,15 @@ __global__ void __launch_bounds__(BT, 1024 / BT)
             for (int r = r0; r < r1; r++, p += 32) sum = O::add(sum, *p);
             O::put(S0, S1, vp, sum);
         }
+        if constexpr (!REG)
+            for (int v = tid + BT; v < n; v += BT) {
+                const int q0 = ld_ro(I.srow + (v >> 5)), q1 = ld_ro(I.srow + (v >> 5) + 1), pub = __ldg(I.perm + v);
+                const V* p = cs + q0 * 32 + (v & 31);
+                V sum = O::splat(T(0));
+#pragma unroll 8
+                for (int r = q0; r < q1; r++, p += 32) sum = O::add(sum, *p);
+                O::put(S0, S1, pub, sum);
+            }
         // the next pass's spins (its buffer is the other one; sy is free: this pass's
         // clause phase has read it)
         if (more) permute(pr + G, b ^ 1);

@@ -14,7 +14,9 @@
 // instance allows it.  Bound by those random sectors of L2, one gather and one store per
 // literal.  One CTA per state with its vectors in global memory, the form before it (still
 // used for the tanh and bias variants, whose clause-weight sum is per CTA), is bound by one
-// SM's L2 latency: four states of N = 1e5, M = 1e6, K = 4 took 6,380 us, 100 us here.
+// SM's L2 latency: four states of N = 1e5, M = 1e6, K = 4 took 6,380 us, 100 us here; 2,176
+// of N = 3800, K = 3 (compact words, clauses out of public order) 1,296 us, 434 us here (618
+// with the clauses taken in the packing's order).
 // Arithmetic as clause_phase / var_phase, lane by lane.
 #pragma once
 
@@ -83,13 +85,16 @@ __global__ void __launch_bounds__(256) row_clause_kernel(RowArgs<T> A) {
     const DevInstance& I = A.I;
     const int g = blockIdx.y;
     const long long it = (long long)blockIdx.x * 256 + threadIdx.x;
-    const int m = (int)(it / R), lb = (int)(it % R) * SUB;
-    if (m >= I.m) return;
+    // public clause order: the accesses to x and dxdt are the coalesced ones, the words those
+    // that follow the packing's clause order (2 L against 2 K accesses a clause)
+    const int j = (int)(it / R), lb = (int)(it % R) * SUB;
+    if (j >= I.m) return;
+    const int m = __ldg(I.icperm + j);
     const T* sy = A.sy + g * A.sy_stride + lb;
     T* cs = A.cs + g * A.cs_stride + lb;
     const T knorm = (T)ldexp(1.0, -I.k);
     const int cnt = A.ns - g * L - lb;  // this thread's lanes below cnt are states
-    const long long at = (A.s0 + (long long)g * L + lb) * A.stride + I.n + __ldg(I.cperm + m);
+    const long long at = (A.s0 + (long long)g * L + lb) * A.stride + I.n + j;
     uint32_t w[KMAX], slot[KMAX];
 #pragma unroll
     for (int q = 0; q < KMAX; q++)
@@ -136,9 +141,9 @@ __global__ void __launch_bounds__(256) row_clause_kernel(RowArgs<T> A) {
                     T prod = T(1);
                     bool first = true;
 #pragma unroll
-                    for (int j = 0; j < KMAX; j++)
-                        if (j != q && (EXACT || j < I.k)) {
-                            prod = first ? f[j][l] : Ar::mul(prod, f[j][l]);
+                    for (int o = 0; o < KMAX; o++)
+                        if (o != q && (EXACT || o < I.k)) {
+                            prod = first ? f[o][l] : Ar::mul(prod, f[o][l]);
                             first = false;
                         }
                     rr = Ar::mul(r[l], prod);
@@ -146,8 +151,8 @@ __global__ void __launch_bounds__(256) row_clause_kernel(RowArgs<T> A) {
                 } else {
                     T temp = kFold ? knorm * km[l] : km[l];
 #pragma unroll
-                    for (int j = 0; j < KMAX; j++)
-                        if (EXACT || j < I.k) temp = Ar::mul(temp, j == q ? T(1) : f[j][l]);
+                    for (int o = 0; o < KMAX; o++)
+                        if (EXACT || o < I.k) temp = Ar::mul(temp, o == q ? T(1) : f[o][l]);
                     rr = Ar::mul(Ar::mul(Ar::mul(T(2), temp), knorm), am[l]);
                 }
                 c.v[l] = neg ? -rr : rr;

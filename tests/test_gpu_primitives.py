@@ -116,3 +116,26 @@ def test_rhs_of_staged_states(n, m, k, batch, shift, dtype, logspace):
     for r in rows:  # a state alone: the same operations
         one = A.get_derivatives(p, xs[r:r + 1].clone(), logspace=logspace).cpu().numpy()
         assert np.array_equal(one[0], got[r])
+
+
+@pytest.mark.parametrize("dtype,logspace", [("float32", True), ("float32", False), ("float64", False)])
+@pytest.mark.parametrize("n,m,k,batch", [(1025, 4200, 3, 3), (1500, 6300, 3, 150), (600, 5200, 4, 2), (2048, 6145, 3, 5),
+                                         (4000, 16500, 3, 11)])
+def test_rhs_of_larger_compact_instances(n, m, k, batch, dtype, logspace):
+    """One FP32 state per staged pass, the one-state kernel, and rows over the whole GPU with
+    clauses out of public order."""
+    lits, lens, _ = make_instance("fast", n, m, k, seed=n + m)
+    p = A.SatProblem.from_arrays(lits, lens)
+    rng = np.random.default_rng(4)
+    x = np.concatenate([rng.uniform(-1, 1, (batch, p.n)), rng.uniform(0.5, 3, (batch, p.m))], axis=1).astype(dtype)
+    xs = torch.from_numpy(x).cuda()
+    got = A.get_derivatives(p, xs, logspace=logspace).cpu().numpy()
+    A.rhs_check(p)
+    rows = [0, batch - 1]
+    want = rhs(lits, lens, x[rows], p.n, p.k, logspace)
+    deg = np.bincount(np.abs(lits) - 1).max()
+    big = np.abs(want).max(axis=1, keepdims=True)
+    assert (np.abs(got[rows] - want) <= (2 * k + deg + 8) * np.finfo(dtype).eps * big).all()
+    for r in rows:  # a state alone: the same operations
+        one = A.get_derivatives(p, xs[r:r + 1].clone(), logspace=logspace).cpu().numpy()
+        assert np.array_equal(one[0], got[r])
