@@ -16,10 +16,14 @@
 //    gather is one logic operation and one load, with no sign flip.
 //  * The clause arithmetic folds its power-of-two scalings (fast_clause), as the
 //    general kernel's FP32 log-space path does.
-//  * Each stage's variable phase also forms the next stage's spin input, and an
-//    accepted step's copy of the clause rows happens in the next stage 1's clause
-//    loop; the error max is an integer redux (lean_max_then) and an accepted step's
-//    next step size is formed in the next stage 1 (settle_h).
+//  * Each stage's variable phase also forms the next stage's spin input (stage 6's the
+//    candidate state, stage 1's input if the step is accepted), the accepted step's copy of
+//    the rows happens in the next stage 1, which reads them anyway, the error max is an
+//    integer redux with one barrier (lean_max), and an accepted step's division and next step
+//    size are formed in the next stage 1 (settle_h).  With two barriers and a division in
+//    the reduction and a pass of its own for the copy, 512 trajectories of N = 1000, M = 4250,
+//    300 steps, took 16.4 ms, 15.6 so.  The parts forms keep those (FP64 5 to 8% slower without:
+//    at 64 registers the same changes spill).
 //  * Literal words are blocked by 32 clauses ([m / 32][q][m % 32]), so a clause's K
 //    words are loads at immediate offsets from one pointer that advances once per
 //    clause, and a warp's 32 clauses load each word as one 128-byte line.
@@ -206,11 +210,10 @@ __device__ __forceinline__ Row6<typename R::Val> load_row(typename R::Ref r) {
     }
     return o;
 }
-// A clause row at stage 1: after an accepted step its new state still sits in slot 2
-// (the accepted step's copy of the clause rows is done here, by the owning thread,
-// where the row is read anyway).
+// A row at stage 1: after an accepted step its new state still sits in slot 2 (the
+// accepted step's copy is done here, by the owning thread, where the row is read anyway).
 template <int S, typename R>
-__device__ __forceinline__ Row6<typename R::Val> load_clause_row(typename R::Ref r, bool from_candidate) {
+__device__ __forceinline__ Row6<typename R::Val> load_moved_row(typename R::Ref r, bool from_candidate) {
     if constexpr (S == 1) {
         if (from_candidate) {
             Row6<typename R::Val> o;
@@ -389,6 +392,16 @@ __device__ __forceinline__ double lean_max_then(double em, uint32_t*, double* re
     return red_d[33];
 }
 
+// The FP32 max with one barrier: after it every warp reduces the warps' maxima for itself.
+__device__ __forceinline__ double lean_max(float em, uint32_t* red_u) {
+    const uint32_t v = __reduce_max_sync(0xffffffffu, __float_as_uint(em));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) red_u[warp] = v;
+    __syncthreads();
+    return (double)__uint_as_float(
+        __reduce_max_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? red_u[lane] : 0u));
+}
+
 __device__ __forceinline__ int ld_relaxed(const int* p) {
     int v;
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -409,7 +422,7 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
     __shared__ double red_d[36];
     __shared__ int red_i[33];
     __shared__ uint32_t red_u[32];
-    __shared__ int s_unit, s_flag;
+    __shared__ int s_unit, s_flag, s_quit;
     const Grp<1> g;
     const int tid = threadIdx.x, nt = blockDim.x;
     const uint32_t sm0 = (uint32_t)__cvta_generic_to_shared(smem_raw);
@@ -482,9 +495,12 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
         bool h_pending = false;
         const int pow_tid = nt >= 64 ? nt - 32 : 0;
         auto settle_h = [&]() {
-            if (h_pending && tid == pow_tid)
-                red_d[34] = e_acc > ck::ERRCON ? __dmul_rn(__dmul_rn(ck::SAFETY, h_acc), pow(e_acc, ck::PGROW))
-                                               : __dmul_rn(5.0, h_acc);
+            if (h_pending && tid == pow_tid) {
+                // the all-shared form leaves the accepted attempt's division to this thread too
+                const double e = PARTS ? e_acc : __ddiv_rn(e_acc, P.eps);
+                red_d[34] = e > ck::ERRCON ? __dmul_rn(__dmul_rn(ck::SAFETY, h_acc), pow(e, ck::PGROW))
+                                           : __dmul_rn(5.0, h_acc);
+            }
         };
         auto take_h = [&]() {
             if (h_pending) hnext = red_d[34];
@@ -494,13 +510,15 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
         // One RHS evaluation at stage S; the derivative lands in slot S of the rows, or
         // for S == 6 is consumed at once into the candidate state (slot 2) and the error
         // norm.  The spins' stage input is formed by the variable phase of the stage
-        // before (ready = true; stage 1's by the accepted step's copy), or here.
+        // before (ready = true; all shared: stage 6's puts the candidate state, which is stage
+        // 1's input if the step is accepted, and the error max's barrier stands for this one;
+        // parts: the accepted step's copy), or here.
         auto eval = [&](auto stage, T hT, T h0T, T& em, bool ready) {
             constexpr int S = decltype(stage)::value;
             if (!ready)
                 for (int v = tid; v < n; v += nt)
                     put_spin(v, row_input<S>(load_row<S, R>(rs.at(v)), hT));
-            g.sync();
+            if (PARTS || S > 1 || !ready) g.sync();
             if constexpr (PARTS) {
                 const int np = I.nparts, ns1 = ((n + 31) >> 5) + 1;
                 for (int pp = 0; pp < np; pp++) {
@@ -508,7 +526,7 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                     const uint32_t* lp = I.plit + lean_word_index(c0 + tid, 0, K);
                     typename R::Ref ra = rs.at(cb + c0 + tid);
                     for (int c = c0 + tid; c < c1; c += nt, lp += (size_t)nt * K, ra = R::advance(ra, nt)) {
-                        const auto o = load_clause_row<S, R>(ra, ready);
+                        const auto o = load_moved_row<S, R>(ra, ready);
                         const T d = part_clause<K>(sb, cs0, lp, weight(row_input<S>(o, hT)), duc);
                         if constexpr (S < 6) {
                             R::st(ra, S, d);
@@ -578,7 +596,7 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
             const uint32_t* lp = I.flit + lean_word_index(tid, 0, K);
             typename R::Ref ra = rs.at(cb + tid);
             for (int c = tid; c < m; c += nt, lp += (size_t)nt * K, ra = R::advance(ra, nt)) {
-                const auto o = load_clause_row<S, R>(ra, ready);
+                const auto o = load_moved_row<S, R>(ra, ready);
                 const T d = fast_clause<K>(sb, mask, cs0, lp, weight(row_input<S>(o, hT)), duc);
                 if constexpr (S < 6) {
                     R::st(ra, S, d);
@@ -595,7 +613,7 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                 const int r0 = ld_ro(I.srow + g32), r1 = ld_ro(I.srow + g32 + 1);
                 uint32_t p = cs0 + 4u * (uint32_t)(r0 * 32 + (v & 31));
                 const typename R::Ref r = rs.at(v);
-                Row6<T> o = load_row<S, R>(r);  // what the next stage's input (or stage 6) reads
+                Row6<T> o = load_moved_row<S, R>(r, ready);  // what the next stage's input (or stage 6) reads
                 T sum = T(0);
 #pragma unroll 8
                 for (int k = r0; k < r1; k++, p += 128u) sum = sum + lds(p);
@@ -605,14 +623,16 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                     put_spin(v, row_input<S + 1>(o, S == 1 ? (T)hnext : hT));
                 } else {
                     em = fmax(em, rk_err_ratio(o.x, o.k1, o.k3, o.k4, o.k5, sum, hT, h0T, false));
-                    R::st(r, 2, rk_new<T>(o.x, o.k1, o.k3, o.k4, sum, hT));
+                    const T xn = rk_new<T>(o.x, o.k1, o.k3, o.k4, sum, hT);
+                    R::st(r, 2, xn);
+                    put_spin(v, xn);
                 }
             }
         };
 
         double t = 0.0, hdid = 0.0;
-        // after an accepted step: the spins hold its state (stage 1's input) and the clause
-        // rows' state is still in slot 2 until the next stage 1 moves it
+        // after an accepted step: the spins hold its state (stage 1's input) and the rows'
+        // state is still in slot 2 until the next stage 1 moves it
         bool s1_ready = false;
         int steps = 0, attempts = 0, rhs = 0, viol = -1, minviol = INT_MAX;
         int status = SAT_UNKNOWN;
@@ -623,11 +643,11 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
             for (int b = 0; b < P.batch; b++) {
                 T dummy = T(0);
                 eval(std::integral_constant<int, 1>{}, T(0), T(0), dummy, s1_ready);
-                s1_ready = false;  // the clause rows' copy is done
+                s1_ready = false;  // the rows' copy is done
                 rhs++;
                 const double h0 = hnext;
                 const T h0T = (T)h0;
-                double h = hnext, ermax = 0.0;
+                double h = hnext;
                 bool retry = false;  // a retry's stage-2 input uses the smaller step
                 while (true) {
                     const T hT = (T)h;
@@ -643,18 +663,34 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                     eval(std::integral_constant<int, 6>{}, hT, h0T, em, true);
                     rhs += 5;
                     attempts++;
-                    ermax = lean_max_then(em, red_u, red_d, [&](double emax) {
-                        const double e = __ddiv_rn(emax, P.eps);
-                        if (e > 1.0)  // rejected: the retry's step size now (accepted: settle_h)
-                            red_d[34] = fmax(__dmul_rn(__dmul_rn(ck::SAFETY, h), pow(e, ck::PSHRNK)),
-                                             __dmul_rn(ck::HFACTOR, h));
-                        const bool quit = other_solved != 0 || (P.deadline && globaltimer_ns() >= deadline);
-                        red_d[35] = quit ? 1.0 : 0.0;
-                        return e;
-                    });
-                    if (red_d[35] != 0.0) { interrupted = true; break; }
-                    if (ermax <= 1.0) {
+                    bool accepted;
+                    if constexpr (PARTS) {
+                        const double ermax = lean_max_then(em, red_u, red_d, [&](double emax) {
+                            const double e = __ddiv_rn(emax, P.eps);
+                            if (e > 1.0)  // rejected: the retry's step size now (accepted: settle_h)
+                                red_d[34] = fmax(__dmul_rn(__dmul_rn(ck::SAFETY, h), pow(e, ck::PSHRNK)),
+                                                 __dmul_rn(ck::HFACTOR, h));
+                            s_quit = other_solved != 0 || (P.deadline && globaltimer_ns() >= deadline);
+                            return e;
+                        });
+                        accepted = ermax <= 1.0;
                         e_acc = ermax;
+                    } else {
+                        // one barrier: emax / eps, rounded to nearest, is above 1 exactly when
+                        // emax > eps, so the division can wait (settle_h; rejected: thread 0)
+                        if (tid == 0) s_quit = other_solved != 0 || (P.deadline && globaltimer_ns() >= deadline);
+                        const double emax = lean_max(em, red_u);
+                        accepted = emax <= P.eps;
+                        e_acc = emax;
+                        if (!accepted && !s_quit) {
+                            if (tid == 0)
+                                red_d[34] = fmax(__dmul_rn(__dmul_rn(ck::SAFETY, h), pow(__ddiv_rn(emax, P.eps), ck::PSHRNK)),
+                                                 __dmul_rn(ck::HFACTOR, h));
+                            g.sync();
+                        }
+                    }
+                    if (s_quit) { interrupted = true; break; }
+                    if (accepted) {
                         h_acc = h;
                         h_pending = true;
                         break;
@@ -667,24 +703,24 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
                 hdid = h;
                 t = __dadd_rn(t, h);
                 taken++;
-                // accept: the candidate state (slot 2) becomes the state, each element by
-                // the thread that owns it in the stage loops; the spins are also the next
-                // stage 1's input.  The clause rows follow in that stage's clause loop.
-                for (int v = tid; v < n; v += nt) {
-                    const typename R::Ref r = rs.at(v);
-                    const T xn = R::ld(r, 2);
-                    R::st(r, 0, xn);
-                    put_spin(v, xn);
-                }
+                // accept: the candidate state (slot 2; all shared: the spins too) becomes the
+                // state; the rows are moved by the next stage 1, in the parts forms the variables'
+                // here, where the spins are put as well
+                if constexpr (PARTS)
+                    for (int v = tid; v < n; v += nt) {
+                        const typename R::Ref r = rs.at(v);
+                        const T xn = R::ld(r, 2);
+                        R::st(r, 0, xn);
+                        put_spin(v, xn);
+                    }
                 s1_ready = true;
             }
             if (underflow) { status = SAT_UNDERFLOW; break; }
             steps += taken;
             if (interrupted) { status = SAT_ODE_INTERRUPTED; break; }
 
-            // CpuSat::GetClauseViolationCount on the accepted state
-            for (int v = tid; v < n; v += nt) sts(sb + VB * (uint32_t)v, R::ld(rs.at(v), 0));
-            g.sync();
+            // CpuSat::GetClauseViolationCount on the accepted state, which the spins hold
+            if constexpr (PARTS) g.sync();
             int cnt = 0;
             {
                 const uint32_t* lp = (PARTS ? I.plit : I.flit) + lean_word_index(tid, 0, K);
@@ -735,9 +771,10 @@ __global__ void __launch_bounds__(1024, 1) solve_kernel_fast(SolveParams P) {
 
         // write back the final state in the public layout
         g.sync();
-        for (int i = tid; i < n; i += nt) G[i] = R::ld(rs.at(__ldg(I.iperm + i)), 0);
+        const int slot = s1_ready ? 2 : 0;
+        for (int i = tid; i < n; i += nt) G[i] = R::ld(rs.at(__ldg(I.iperm + i)), PARTS ? 0 : slot);
         for (int j = tid; j < m; j += nt) {
-            const T a = R::ld(rs.at(cb + __ldg(icp + j)), s1_ready ? 2 : 0);
+            const T a = R::ld(rs.at(cb + __ldg(icp + j)), slot);
             if constexpr (LOGA) G[n + j] = exp2f(a);
             else G[n + j] = a;
         }
