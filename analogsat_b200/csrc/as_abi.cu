@@ -1061,7 +1061,10 @@ int32_t as_solver_set_wall_budget(as_solver* s, double v) {
 }
 int32_t as_solver_set_stop_on_first(as_solver* s, int32_t f) {
     if (!s) return fail(AS_ERR_BAD_INPUT, "null solver");
-    s->stop_on_first = f ? 1 : 0; s->groups_dirty = true; s->invalidate();
+    if (s->stop_on_first == (f ? 1 : 0)) return AS_OK;
+    s->stop_on_first = f ? 1 : 0;
+    s->groups_dirty = true;  // the queue order depends on it
+    s->invalidate();
     return AS_OK;
 }
 int32_t as_solver_set_track_best(as_solver* s, int32_t f) {
@@ -1085,6 +1088,7 @@ int plan_units(as_solver* s, const int32_t* problem_index, int num_traj) {
     if (num_traj == s->num_traj && s->states.p &&
         std::equal(problem_index, problem_index + num_traj, s->traj_problem.begin()))
         return AS_OK;
+    AS_CUDA(cudaStreamSynchronize(s->stream));  // a solve in flight still uses the buffers
     s->num_traj = num_traj;
     s->traj_problem.assign(problem_index, problem_index + num_traj);
     s->traj_off.resize(num_traj);
@@ -1110,9 +1114,24 @@ int plan_units(as_solver* s, const int32_t* problem_index, int num_traj) {
     return AS_OK;
 }
 
+// The unit tables, by the solver's own stream: a copy on the default stream is not ordered
+// with the kernels on this one, which does not wait for it.
+int upload_unit_tables(as_solver* s, const std::vector<int>& ui, const std::vector<long long>& us,
+                       const std::vector<long long>& ub) {
+    AS_CUDA(cudaMemcpyAsync(s->unit_inst.p, ui.data(), sizeof(int) * ui.size(), cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaMemcpyAsync(s->unit_state.p, us.data(), sizeof(long long) * us.size(), cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaMemcpyAsync(s->unit_bits.p, ub.data(), sizeof(long long) * ub.size(), cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaStreamSynchronize(s->stream));  // the host vectors may go
+    return AS_OK;
+}
+
 // Pick the launch shape of every problem (smallest CTA that holds it, or the forced
-// shape), order the trajectories by (shape, problem) and upload the unit tables.
+// shape), order the trajectories by (shape, problem) and upload the unit tables.  An
+// asynchronous solve still in flight reads the tables and works in the slabs, so it is
+// waited for first: the solver's stream follows every solve, those on a caller's stream too
+// (ev_out).
 int build_groups(as_solver* s) {
+    AS_CUDA(cudaStreamSynchronize(s->stream));
     const auto& vs = variants();
     const int np = (int)s->problems.size();
     const int num_traj = s->num_traj;
@@ -1275,9 +1294,8 @@ int build_groups(as_solver* s) {
     }
     if (s->groups.size() + 1 > s->queue.bytes / sizeof(int))
         AS_CUDA(s->queue.alloc(sizeof(int) * (s->groups.size() + 1)));
-    AS_CUDA(cudaMemcpy(s->unit_inst.p, ui.data(), sizeof(int) * num_traj, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(s->unit_state.p, us.data(), sizeof(long long) * num_traj, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(s->unit_bits.p, ub.data(), sizeof(long long) * num_traj, cudaMemcpyHostToDevice));
+    const int r = upload_unit_tables(s, ui, us, ub);
+    if (r) return r;
     s->groups_dirty = false;
     s->invalidate();
     return AS_OK;
@@ -1511,8 +1529,9 @@ int stream_lists(as_solver* s, int p) {
     AS_CUDA(P.vstart[p]->alloc(sizeof(int) * std::max<size_t>(split.size(), 1)));
     AS_CUDA(P.vpos[p]->alloc(sizeof(int) * pos.size()));
     if (!split.empty())
-        AS_CUDA(cudaMemcpy(P.vstart[p]->p, split.data(), sizeof(int) * split.size(), cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(P.vpos[p]->p, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice));
+        AS_CUDA(cudaMemcpyAsync(P.vstart[p]->p, split.data(), sizeof(int) * split.size(), cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaMemcpyAsync(P.vpos[p]->p, pos.data(), sizeof(int) * pos.size(), cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaStreamSynchronize(s->stream));  // the host vectors may go
     P.nparts[p] = parts;
     P.have_lists[p] = 1;
     return AS_OK;
@@ -1592,13 +1611,10 @@ int stream_plan(as_solver* s) {
         us[u] = s->traj_off[s->order[u]];
         ub[u] = s->traj_bits[s->order[u]];
     }
-    AS_CUDA(cudaMemcpy(P.lanes.p, lanes.data(), sizeof(LaneState) * lanes.size(), cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(P.active.p, act.data(), sizeof(int) * P.ngroups, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemset(P.tickets.p, 0, sizeof(int) * 2 * P.ngroups));
-    AS_CUDA(cudaMemcpy(s->unit_inst.p, ui.data(), sizeof(int) * num_traj, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(s->unit_state.p, us.data(), sizeof(long long) * num_traj, cudaMemcpyHostToDevice));
-    AS_CUDA(cudaMemcpy(s->unit_bits.p, ub.data(), sizeof(long long) * num_traj, cudaMemcpyHostToDevice));
-    return AS_OK;
+    AS_CUDA(cudaMemcpyAsync(P.lanes.p, lanes.data(), sizeof(LaneState) * lanes.size(), cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaMemcpyAsync(P.active.p, act.data(), sizeof(int) * P.ngroups, cudaMemcpyHostToDevice, s->stream));
+    AS_CUDA(cudaMemsetAsync(P.tickets.p, 0, sizeof(int) * 2 * P.ngroups, s->stream));
+    return upload_unit_tables(s, ui, us, ub);
 }
 
 // The clause and variable kernels of stage S: compiled for the stage where the clause
