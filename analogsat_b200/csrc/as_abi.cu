@@ -20,6 +20,7 @@
 #include "../../include/analogsat_b200.h"
 #include "as_ingest.h"
 #include "as_adjoint.cuh"
+#include "as_devbuf.h"
 #include "as_fast.cuh"
 #include "as_kernels.cuh"
 #include "as_problem.h"
@@ -50,27 +51,6 @@ int fail(int code, const std::string& msg) {
         if (e_ != cudaSuccess)                                                          \
             return fail(AS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
-
-struct DevBuf {
-    void* p = nullptr;
-    size_t bytes = 0;
-    ~DevBuf() { release(); }
-    void release() {
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-    }
-    cudaError_t alloc(size_t b) {
-        if (b <= bytes && p) return cudaSuccess;
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(b, 16));
-        if (e == cudaSuccess) bytes = b;
-        return e;
-    }
-    template <typename T> T* as() const { return static_cast<T*>(p); }
-};
 
 // Device copy of one or more packed instances in a single pool.
 struct DevicePool {
@@ -407,7 +387,6 @@ struct as_problem {
     struct Prepared { const void* fn; int dev; size_t smem; int occ; };
     std::vector<Prepared> prepared_;
     DevBuf rhs_status;        // set by a device RHS whose bulk copy timed out (as_rhs_check)
-    int rhs_status_dev = -1;  // device holding rhs_status
 
     int tanh = 0;       // CTDS variant (ISat implementation) and its parameters
     double q = 1.1, b = 0.0;
@@ -769,10 +748,9 @@ int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename St
     const int grid = std::max(1, std::min(passes, D.sms * occ));
     // bulk stores need dxdt congruent with x mod 16 bytes (same staging offsets)
     const int bulk_out = ((reinterpret_cast<uintptr_t>(x) - reinterpret_cast<uintptr_t>(d)) & 15u) == 0;
-    if (p->rhs_status_dev != dev) {
+    if (!p->rhs_status.holds(sizeof(int), dev)) {
         AS_CUDA(p->rhs_status.alloc(sizeof(int)));
         AS_CUDA(cudaMemset(p->rhs_status.p, 0, sizeof(int)));
-        p->rhs_status_dev = dev;
     }
     fn<<<grid, BT, smem, st>>>(p->dev[layout].host_inst[0], x, d, ns, (long long)(q.n + q.m), bulk_out,
                                p->rhs_status.as<int>());
@@ -934,13 +912,14 @@ int32_t as_rhs_f32(as_problem* p, const float* x, float* dxdt, int32_t num_state
 int32_t as_rhs_check(as_problem* p, void* stream) {
     if (!p) return fail(AS_ERR_BAD_INPUT, "as_rhs_check: null problem");
     AS_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    if (p->rhs_status_dev < 0) return AS_OK;  // no bulk-copy RHS has run
+    const int on = p->rhs_status.dev;
+    if (on < 0) return AS_OK;  // no bulk-copy RHS has run
     int dev = 0, word = 0;
     AS_CUDA(cudaGetDevice(&dev));
-    if (dev != p->rhs_status_dev) AS_CUDA(cudaSetDevice(p->rhs_status_dev));
+    if (dev != on) AS_CUDA(cudaSetDevice(on));
     cudaError_t e = cudaMemcpy(&word, p->rhs_status.p, sizeof(int), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && word) e = cudaMemset(p->rhs_status.p, 0, sizeof(int));
-    if (dev != p->rhs_status_dev) cudaSetDevice(dev);
+    if (dev != on) cudaSetDevice(dev);
     if (e != cudaSuccess) return fail(AS_ERR_CUDA, std::string("as_rhs_check: ") + cudaGetErrorString(e));
     if (word)
         return fail(AS_ERR_TIMEOUT, "as_rhs_f32: a bulk copy did not complete within 2 s; the states "
