@@ -52,6 +52,55 @@ int fail(int code, const std::string& msg) {
             return fail(AS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// Scratch of a problem's standalone primitives, grown on demand.  They are asynchronous on
+// the caller's stream and share it, so each waits for the one before (an event; about a
+// microsecond, against the 100 of the calls that need scratch).  A capture takes no part in
+// that: it neither waits nor is waited for, and the buffer that its graph addresses is
+// kept when a later call outgrows it.
+struct Workspace {
+    DevBuf buf;
+    std::vector<std::unique_ptr<DevBuf>> captured;  // outgrown, addressed by captured graphs
+    cudaEvent_t done = nullptr;                     // end of the last use outside a capture
+    int done_dev = -1;
+    bool capturing = false, in_graph = false;
+
+    ~Workspace() { if (done) cudaEventDestroy(done); }
+    // `bytes` of scratch on the current device for work queued on `st` until end(st).
+    int begin(size_t bytes, cudaStream_t st) {
+        cudaStreamCaptureStatus status;
+        AS_CUDA(cudaStreamIsCapturing(st, &status));
+        capturing = status != cudaStreamCaptureStatusNone;
+        int dev = 0;
+        AS_CUDA(cudaGetDevice(&dev));
+        if (buf.holds(bytes, dev)) {
+            if (done && !capturing) AS_CUDA(cudaStreamWaitEvent(st, done, 0));
+        } else {
+            if (done) AS_CUDA(cudaEventSynchronize(done));
+            if (done && done_dev != dev) {
+                cudaEventDestroy(done);
+                done = nullptr;
+            }
+            if (in_graph) {
+                captured.emplace_back(new DevBuf());
+                captured.back()->take(buf);
+                in_graph = false;
+            }
+            AS_CUDA(buf.alloc(bytes));
+        }
+        in_graph |= capturing;
+        return AS_OK;
+    }
+    int end(cudaStream_t st) {
+        if (capturing) return AS_OK;
+        if (!done) {
+            AS_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+            AS_CUDA(cudaGetDevice(&done_dev));
+        }
+        AS_CUDA(cudaEventRecord(done, st));
+        return AS_OK;
+    }
+};
+
 // Device copy of one or more packed instances in a single pool.
 struct DevicePool {
     int device = -1;
@@ -381,7 +430,7 @@ struct as_problem {
     bool have_[3] = {false, false, false};
     std::mutex mu_;
     DevicePool dev[3];        // lazily uploaded for the device primitives
-    DevBuf slab[3];           // per-CTA storage of the global-storage primitives
+    Workspace work[3];        // scratch of the primitives of instances beyond one SM
     // Kernels of the standalone primitives that have been prepared for this problem (shared
     // memory limit raised, occupancy asked): the instance fixes the shape of each.
     struct Prepared { const void* fn; int dev; size_t smem; int occ; };
@@ -760,9 +809,8 @@ int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename St
 }
 
 // States of an instance that fits no SM (as_rows.cuh): chunks of state groups, three
-// kernels per chunk.  The rows of a chunk's groups live in a slab owned by the problem
-// handle (grown on demand; calls on one handle must not overlap), about 64 MB -- half of
-// L2 -- or one group's where that is more.
+// kernels per chunk.  The rows of a chunk's groups live in the problem's scratch, about
+// 64 MB -- half of L2 -- or one group's where that is more.
 template <typename T, bool LOGA, int KMAX, bool EXACT, int SUB, int R>
 int launch_rhs_rows(as_problem* p, int prec, const T* x, T* d, int ns, cudaStream_t st) {
     constexpr int L = SUB * R;
@@ -777,8 +825,9 @@ int launch_rhs_rows(as_problem* p, int prec, const T* x, T* d, int ns, cudaStrea
     const long long group_bytes = (A.sy_stride + A.cs_stride) * (long long)sizeof(T);
     const int groups = (ns + L - 1) / L;
     const int chunk = (int)std::max(1ll, std::min({(long long)groups, 65535ll, (64ll << 20) / group_bytes}));
-    AS_CUDA(p->slab[prec].alloc((size_t)chunk * group_bytes));
-    A.sy = p->slab[prec].template as<T>();
+    int r = p->work[prec].begin((size_t)chunk * group_bytes, st);
+    if (r) return r;
+    A.sy = p->work[prec].buf.template as<T>();
     A.cs = A.sy + chunk * A.sy_stride;
     for (int g = 0; g < groups; g += chunk) {
         A.s0 = (long long)g * L;
@@ -789,8 +838,9 @@ int launch_rhs_rows(as_problem* p, int prec, const T* x, T* d, int ns, cudaStrea
             <<<dim3((unsigned)(((long long)R * A.I.m + 255) / 256), gy), 256, 0, st>>>(A);
         row_var_kernel<T, SUB, R><<<dim3((unsigned)(((long long)R * A.I.n + 255) / 256), gy), 256, 0, st>>>(A);
     }
+    r = p->work[prec].end(st);
     AS_CUDA(cudaGetLastError());
-    return AS_OK;
+    return r;
 }
 
 template <typename T, bool LOGA, int KMAX, bool EXACT>
@@ -827,12 +877,13 @@ int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
         if ((r = prepare_kernel(p, (const void*)fg, BT, 0, dev, &occ))) return r;
         const int grid = std::max(1, std::min(ns, D.sms * std::max(occ, 1)));
         const long long slab_stride = (long long)((vals + 63) / 64 * 64);
-        AS_CUDA(p->slab[prec].alloc((size_t)grid * slab_stride * sizeof(T)));
-        fg<<<grid, BT, 0, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, p->slab[prec].template as<T>(),
+        if ((r = p->work[prec].begin((size_t)grid * slab_stride * sizeof(T), st))) return r;
+        fg<<<grid, BT, 0, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, p->work[prec].buf.template as<T>(),
                                 slab_stride);
+        r = p->work[prec].end(st);
     }
     AS_CUDA(cudaGetLastError());
-    return AS_OK;
+    return r;
 }
 
 template <typename T, bool LOGA>
@@ -875,15 +926,16 @@ int launch_viol(as_problem* p, const T* x, int* c, int ns, cudaStream_t st) {
         fn<<<grid, grid > sms ? 256 : 1024, smem, st>>>(I, x, c, ns, stride, per);
     } else {
         const int groups = (ns + 31) / 32, gy = std::min(groups, 65535);
-        AS_CUDA(p->slab[prec].alloc(4 * (size_t)groups * ((size_t)I.n + 1)));
-        uint32_t* gmask = p->slab[prec].template as<uint32_t>();
+        if ((r = p->work[prec].begin(4 * (size_t)groups * ((size_t)I.n + 1), st))) return r;
+        uint32_t* gmask = p->work[prec].buf.template as<uint32_t>();
         viol_mask_kernel<T><<<dim3((I.n + 256) / 256, gy), 256, 0, st>>>(I, x, c, gmask, ns, stride);
         // about eight CTAs per SM over all groups, at least four clauses per thread
         const int slices = std::max(1, std::min((I.m + 1023) / 1024, (8 * sms + gy - 1) / gy));
         viol_count_kernel<KMAX, EXACT><<<dim3(slices, gy), 256, 0, st>>>(I, c, gmask, ns);
+        r = p->work[prec].end(st);
     }
     AS_CUDA(cudaGetLastError());
-    return AS_OK;
+    return r;
 }
 
 template <typename T>

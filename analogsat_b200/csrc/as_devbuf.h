@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <utility>
 
 namespace asb {
 
@@ -49,6 +50,13 @@ struct DevBuf {
             p = nullptr;
         }
         return e;
+    }
+    // The other's buffer, which is left empty.
+    void take(DevBuf& o) {
+        release();
+        std::swap(p, o.p);
+        std::swap(bytes, o.bytes);
+        std::swap(dev, o.dev);
     }
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };

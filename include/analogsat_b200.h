@@ -123,7 +123,14 @@ int32_t as_problem_set_model(as_problem* p, int32_t model, double q);
 int32_t as_problem_set_bias(as_problem* p, double b);
 int32_t as_problem_get_model(const as_problem* p, int32_t* model, double* q, double* b);
 
-/* ---- device primitives (ISat, AnalogSAT/solver/ISat.h:31-87) -------------- */
+/* ---- device primitives (ISat, AnalogSAT/solver/ISat.h:31-87) --------------
+ * as_rhs_* and as_violations_* are asynchronous on `stream`; calls on one problem from
+ * several streams may be queued without waiting in between.  For instances that no SM
+ * holds they share scratch memory of the problem, and each waits on the GPU for the one
+ * queued before.  A call inside a stream capture takes no part in that order: replays of
+ * its graph must not overlap other such calls on the problem.  The first call of its
+ * kind (and, beyond one SM, the one with the most states) belongs before the capture,
+ * since it allocates. */
 
 /* ISat::GetDerivatives over `num_states` states at once (CpuSat.cpp:65-94,
  * CudaSat1.cu:501-531).  x and dxdt are DEVICE pointers to num_states public-layout
