@@ -403,7 +403,9 @@ int shared_cta_threads(size_t smem_bytes, int bt, int device, int* out) {
 // a warp without clauses for the step size's pow().  Never fewer threads than `bt`, the size
 // for a full GPU.  us per RHS of a trajectory, 16 trajectories, bt threads and so: N = 50
 // FP64 1.55 -> 1.09, FP32 0.89 -> 0.61; N = 200 FP32 1.01 -> 0.89; 300 of N = 50 FP64 1.54 ->
-// 1.17 (before the FP64 redux of the error max).
+// 1.17 (before the FP64 redux of the error max).  Not for instances with the bias term: it
+// sums the clause weights over the CTA's threads, so the CTA size is part of its rounding
+// and has to follow from the instances alone.
 int few_units_threads(int bt, int m, int units, int sms) {
     const int per = (units + sms - 1) / sms;
     const int share = 1024 / per / 32 * 32, one = (m + 31) / 32 * 32 + 32;
@@ -1243,11 +1245,13 @@ int build_groups(as_solver* s) {
         const int vi = pv[pi[s->order[u]]];
         const Variant& v = vs[vi];
         int e = u, bt = 64, mmax = 1;
+        bool bias = false;
         size_t vals = 0, sbytes = 0;
         while (e < num_traj && pv[pi[s->order[e]]] == vi) {
             const auto& q = s->problems[pi[s->order[e]]];
             bt = std::max(bt, preferred_bt(q));
             mmax = std::max(mmax, q.m);
+            bias |= q.b > 0.0;
             vals = std::max(vals, solver_slab_values(v, q));
             sbytes = std::max(sbytes, solver_smem(v, q));
             e++;
@@ -1271,7 +1275,7 @@ int build_groups(as_solver* s) {
         if (!v.gs || v.lean) {
             const int r = shared_cta_threads(sbytes, bt, s->device, &sm_bt);
             if (r) return r;
-            sm_bt = few_units_threads(sm_bt, mmax, e - u, s->sm_count);
+            if (!bias) sm_bt = few_units_threads(sm_bt, mmax, e - u, s->sm_count);
         }
         G.bt = s->forced_bt ? s->forced_bt : (v.gs && !v.lean ? (v.cl > 1 ? 1024 : gs_bt) : sm_bt);
         G.smem = sbytes;
