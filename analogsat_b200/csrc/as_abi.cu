@@ -412,6 +412,14 @@ int few_units_threads(int bt, int m, int units, int sms) {
     return std::max(bt, std::min(share, one));
 }
 
+// The CTA size of a shared-memory or lean launch: `units` trajectories of instances whose
+// largest takes smem_bytes, bt threads on a full GPU and m clauses.
+int solver_threads(size_t smem_bytes, int bt, int m, bool bias, int units, int sms, int device, int* out) {
+    const int r = shared_cta_threads(smem_bytes, bt, device, out);
+    if (!r && !bias) *out = few_units_threads(*out, m, units, sms);
+    return r;
+}
+
 __global__ void stamp_deadline_kernel(unsigned long long* out, unsigned long long budget_ns) {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1273,9 +1281,8 @@ int build_groups(as_solver* s) {
         // the largest CTA (more warps to hide the clause phase's latencies)
         int sm_bt = bt;
         if (!v.gs || v.lean) {
-            const int r = shared_cta_threads(sbytes, bt, s->device, &sm_bt);
+            const int r = solver_threads(sbytes, bt, mmax, bias, e - u, s->sm_count, s->device, &sm_bt);
             if (r) return r;
-            if (!bias) sm_bt = few_units_threads(sm_bt, mmax, e - u, s->sm_count);
         }
         G.bt = s->forced_bt ? s->forced_bt : (v.gs && !v.lean ? (v.cl > 1 ? 1024 : gs_bt) : sm_bt);
         G.smem = sbytes;
@@ -2209,12 +2216,12 @@ int32_t as_solver_solve_noalloc(as_solver* s, int32_t problem_index, int32_t num
     if (!v)
         return fail(AS_ERR_UNSUPPORTED, "as_solver_solve_noalloc: the instance does not fit one SM's shared "
                                         "memory (only shared-memory launches need no device buffers)");
+    const size_t smem = solver_smem(*v, q);
     int bt = s->forced_bt;
-    if (!bt) {
-        r = shared_cta_threads(solver_smem(*v, q), std::max(64, preferred_bt(q)), s->device, &bt);
+    if (!bt) {  // as build_groups does for a call of num_traj trajectories
+        r = solver_threads(smem, std::max(64, preferred_bt(q)), q.m, q.b > 0.0, num_traj, s->sm_count, s->device, &bt);
         if (r) return r;
     }
-    const size_t smem = solver_smem(*v, q);
     cudaStream_t st = (cudaStream_t)stream;
 
     noalloc_prepare_kernel<<<std::max(1, std::min(s->sm_count, (num_traj + 255) / 256)), 256, 0, st>>>(
@@ -2251,6 +2258,11 @@ int32_t as_solver_solve_noalloc(as_solver* s, int32_t problem_index, int32_t num
     e = cudaLaunchKernel((const void*)v->fn, dim3(std::min(num_traj, s->sm_count * occ)), dim3(bt), args,
                          smem, st);
     if (e != cudaSuccess) return fail(AS_ERR_CUDA, std::string("solve launch: ") + cudaGetErrorString(e));
+    s->last_bt = bt;
+    s->last_ctas = std::min(num_traj, s->sm_count * occ);
+    s->last_smem = (int)smem;
+    s->last_occ = occ;
+    s->last_kernel = v->name();
     return AS_OK;
 }
 

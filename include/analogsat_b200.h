@@ -257,8 +257,9 @@ int32_t as_solver_write_result(as_solver* s, int32_t traj, const char* path);
 int32_t as_solver_append_perf(as_solver* s, int32_t traj, const char* path, const char* sample,
                               const char* solver_name);
 
-/* Launch shape of the last solve's final launch group: threads per CTA, CTAs
- * launched, dynamic shared memory per CTA and resident CTAs per SM. */
+/* Launch shape of the last solve's final launch group (as_solver_solve_noalloc has
+ * one group): threads per CTA, CTAs launched, dynamic shared memory per CTA and
+ * resident CTAs per SM. */
 int32_t as_solver_get_launch_shape(as_solver* s, int32_t* threads, int32_t* ctas, int32_t* smem_bytes,
                                    int32_t* ctas_per_sm);
 /* Force the CTA size (a multiple of 32 in [32, 1024]) of the next solves; 0 restores
@@ -346,7 +347,8 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
  *    (N=1000/M=4250 in FP32 does): the global-storage and streamed modes need
  *    device buffers, so as_solver_set_storage_mode is not consulted and a larger
  *    instance fails with AS_ERR_UNSUPPORTED.  The CTA size is the one
- *    as_solver_solve picks for the same instance (or as_solver_force_threads').
+ *    as_solver_solve picks for the same instance and number of trajectories (or
+ *    as_solver_force_threads').
  *  - The solver's settings apply (epsilon, max time/steps, batch size, wall budget,
  *    stop-on-first); best-assignment tracking is not available here.
  *  - Asynchronous on `stream`; results are valid once the stream reaches this point. */
