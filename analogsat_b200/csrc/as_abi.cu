@@ -482,8 +482,7 @@ struct StreamPlan {
 };
 
 // Device buffers of as_solver_adjoint, kept between calls on one solver (grown on demand;
-// the checkpoint pool and the step tables are given back after a call that needed more
-// than kAdjointKeep bytes of them).
+// one of more than kAdjointKeep bytes is given back after the call, an unsuccessful one too).
 constexpr size_t kAdjointKeep = 1ull << 30;
 struct AdjointPlan {
     DevBuf ui, us, uw, w, hs, off, ns, used, loss, gx, gw, ck, hsc;
@@ -515,9 +514,13 @@ struct AdjointPlan {
         return pageable.data();
     }
     void trim() {
-        for (DevBuf* b : {&ck, &hs, &off})
+        for (DevBuf* b : {&ck, &hs, &off, &w, &gx, &gw, &hsc})
             if (b->bytes > kAdjointKeep) b->release();
     }
+};
+struct AdjointTrim {
+    AdjointPlan& plan;
+    ~AdjointTrim() { plan.trim(); }
 };
 
 struct as_solver {
@@ -2367,9 +2370,10 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     }
     if (!s->ap) s->ap.reset(new AdjointPlan());
     AdjointPlan& A = *s->ap;
+    const AdjointTrim trim{A};
     cudaStream_t st = s->stream;
     AS_CUDA(A.hs.alloc(sizeof(double) * (size_t)nt * max_steps));
-    AS_CUDA(A.off.alloc(sizeof(long long) * (size_t)nt * (max_steps + 1)));
+    AS_CUDA(A.off.alloc(sizeof(long long) * (size_t)nt * ((size_t)max_steps + 1)));
     AS_CUDA(A.ns.alloc(sizeof(int) * (nt + 2)));
     AS_CUDA(A.used.alloc(sizeof(unsigned long long)));
     AS_CUDA(A.loss.alloc(sizeof(double) * nt));
@@ -2390,8 +2394,11 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
         AS_CUDA(A.w.alloc(sizeof(double) * (size_t)std::max<long long>(wtot, 1)));
         AS_CUDA(cudaMemcpyAsync(A.w.p, weights, sizeof(double) * wtot, cudaMemcpyHostToDevice, st));
     }
-    // A first guess of 48 checkpoints per trajectory; the forward pass counts what it needs.
-    if (!A.ck.p) AS_CUDA(A.ck.alloc(vb * (size_t)std::min<long long>(etot * std::min(max_steps + 1, 48), 1ll << 27)));
+    // A first guess of 48 checkpoints per trajectory, without which the forward pass just
+    // counts what it needs: a call whose checkpoints fit the memory left must not fail for it.
+    if (!A.ck.p &&
+        A.ck.alloc(vb * (size_t)std::min<long long>(etot * std::min(max_steps, 47) + etot, 1ll << 27)) != cudaSuccess)
+        cudaGetLastError();
 
     AdjointParams P;
     P.inst = s->pool.inst.as<DevInstance>();
@@ -2454,7 +2461,14 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     const size_t row = sizeof(double) * used_steps;
     if (step_sizes && used_steps > 0) {
         AS_CUDA(A.hsc.alloc(row * nt));
-        AS_CUDA(cudaMemcpy2DAsync(A.hsc.p, row, A.hs.p, sizeof(double) * max_steps, row, nt, cudaMemcpyDeviceToDevice, st));
+        const size_t pitch = sizeof(double) * (size_t)max_steps;
+        if (pitch <= (size_t)INT_MAX) {
+            AS_CUDA(cudaMemcpy2DAsync(A.hsc.p, row, A.hs.p, pitch, row, nt, cudaMemcpyDeviceToDevice, st));
+        } else {  // beyond the pitch that a 2-D copy takes
+            for (int t = 0; t < nt; t++)
+                AS_CUDA(cudaMemcpyAsync(A.hsc.as<double>() + (size_t)t * used_steps, A.hs.as<double>() + (size_t)t * max_steps,
+                                        row, cudaMemcpyDeviceToDevice, st));
+        }
         hs.resize((size_t)nt * used_steps);
     }
     const size_t gxn = (size_t)s->total_values, chunk = std::min<size_t>(gxn, 1u << 24);
@@ -2481,6 +2495,5 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     if (!hs.empty())
         for (int t = 0; t < nt; t++)
             std::copy_n(hs.begin() + (size_t)t * used_steps, ns[t], step_sizes + (size_t)t * max_steps);
-    A.trim();
     return AS_OK;
 }

@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(1024, 1) adj_forward_kernel(AdjointParams P) {
         double t = 0.0, hnext = 1e-9;
         int steps = 0, status = 0;
         double* hs = P.hs + (long long)u * P.max_steps;
-        long long* off = P.ckpt_off + (long long)u * (P.max_steps + 1);
+        long long* off = P.ckpt_off + (long long)u * (P.max_steps + 1ll);
         // room for one checkpoint in the pool (one thread); -1 when it is full
         auto reserve = [&](int s) {
             const long long o = (long long)atomicAdd(P.ckpt_used, (unsigned long long)E);
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(1024, 1) adj_backward_kernel(AdjointParams P) 
         A.init(smem_raw, n, I.m, true, P.weights != nullptr);
         const T knorm = (T)ldexp(1.0, -I.k);
         const double* hs = P.hs + (long long)u * P.max_steps;
-        const long long* off = P.ckpt_off + (long long)u * (P.max_steps + 1);
+        const long long* off = P.ckpt_off + (long long)u * (P.max_steps + 1ll);
         const T* pool = reinterpret_cast<const T*>(P.ckpt);
         const T* xT = pool + off[ns];
         load_weights<T>(I, P, u, A.w);
