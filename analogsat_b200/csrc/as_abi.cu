@@ -241,6 +241,9 @@ struct DevicePool {
         }
         AS_CUDA(cudaMemcpy(inst.p, host_inst.data(), sizeof(DevInstance) * host_inst.size(),
                            cudaMemcpyHostToDevice));
+        // the last bytes may still be on their way from the staging memory, and streams that
+        // do not wait for the default one read the tables next
+        AS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
         device = dev;
         return AS_OK;
     }
@@ -774,11 +777,22 @@ int prepare_kernel(as_problem* p, const void* fn, int bt, size_t smem, int dev, 
     return AS_OK;
 }
 
+// The status word of the staged right-hand side, on the device of its kernels.  It comes with
+// the first tables, so that a problem whose tables are there can be captured.
+int ensure_status(as_problem* p, int dev) {
+    if (p->rhs_status.holds(sizeof(int), dev)) return AS_OK;
+    AS_CUDA(p->rhs_status.alloc(sizeof(int)));
+    AS_CUDA(cudaMemset(p->rhs_status.p, 0, sizeof(int)));
+    return AS_OK;
+}
+
 int ensure_uploaded(as_problem* p, int prec) {
     if (p->host.m == 0 || p->host.k == 0) return fail(AS_ERR_NO_PROBLEM, "SAT problem has not been set");
     int dev = 0;
     AS_CUDA(cudaGetDevice(&dev));
     if (p->dev[prec].device == dev) return AS_OK;
+    const int r = ensure_status(p, dev);
+    if (r) return r;
     std::vector<const PackedProblem*> v{&p->packed(prec)};
     return p->dev[prec].upload(v, dev);
 }
@@ -824,10 +838,7 @@ int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename St
     const int grid = std::max(1, std::min(passes, D.sms * occ));
     // bulk stores need dxdt congruent with x mod 16 bytes (same staging offsets)
     const int bulk_out = ((reinterpret_cast<uintptr_t>(x) - reinterpret_cast<uintptr_t>(d)) & 15u) == 0;
-    if (!p->rhs_status.holds(sizeof(int), dev)) {
-        AS_CUDA(p->rhs_status.alloc(sizeof(int)));
-        AS_CUDA(cudaMemset(p->rhs_status.p, 0, sizeof(int)));
-    }
+    if ((r = ensure_status(p, dev))) return r;
     fn<<<grid, BT, smem, st>>>(p->dev[layout].host_inst[0], x, d, ns, (long long)(q.n + q.m), bulk_out,
                                p->rhs_status.as<int>());
     AS_CUDA(cudaGetLastError());
