@@ -1371,6 +1371,14 @@ int build_groups(as_solver* s) {
     return AS_OK;
 }
 
+// The events that order a caller's stream with the solver's.
+cudaError_t ensure_order_events(as_solver* s) {
+    cudaError_t e = cudaSuccess;
+    if (!s->ev_in) e = cudaEventCreateWithFlags(&s->ev_in, cudaEventDisableTiming);
+    if (e == cudaSuccess && !s->ev_out) e = cudaEventCreateWithFlags(&s->ev_out, cudaEventDisableTiming);
+    return e;
+}
+
 template <typename SRC>
 int set_states_host(as_solver* s, const int32_t* pi, int nt, const SRC* src) {
     if (!s || !src) return fail(AS_ERR_BAD_INPUT, "as_solver_set_states: null argument");
@@ -1845,9 +1853,24 @@ int32_t as_solver_set_states_device(as_solver* s, const int32_t* pi, int32_t nt,
     int r = plan_units(s, pi, nt);
     if (r) return r;
     const size_t vb = s->precision == AS_PREC_F64 ? 8 : 4;
-    AS_CUDA(cudaMemcpyAsync(s->states.p, src, (size_t)s->total_values * vb, cudaMemcpyDeviceToDevice,
-                            stream ? (cudaStream_t)stream : s->stream));
-    if (stream) AS_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    // The copy runs on the solver's stream (behind a solve that still works on the states),
+    // after what the caller's stream has queued (src may still be written there) and
+    // before what it queues later (src may be reused).
+    const cudaStream_t st = stream ? (cudaStream_t)stream : cudaStreamLegacy;
+    AS_CUDA(ensure_order_events(s));
+    if (cudaEventRecord(s->ev_in, st) == cudaSuccess) {
+        AS_CUDA(cudaStreamWaitEvent(s->stream, s->ev_in, 0));
+    } else {  // a stream of another GPU, whose tensor this is
+        cudaGetLastError();
+        AS_CUDA(cudaStreamSynchronize(st));
+    }
+    AS_CUDA(cudaMemcpyAsync(s->states.p, src, (size_t)s->total_values * vb, cudaMemcpyDeviceToDevice, s->stream));
+    if (stream) {
+        AS_CUDA(cudaStreamSynchronize(s->stream));
+    } else {
+        AS_CUDA(cudaEventRecord(s->ev_out, s->stream));
+        AS_CUDA(cudaStreamWaitEvent(st, s->ev_out, 0));
+    }
     return AS_OK;
 }
 
@@ -1892,8 +1915,7 @@ int32_t as_solver_solve_async(as_solver* s, void* stream) {
         // The solve runs on the caller's stream: after the work already queued on the
         // solver's stream (states copied in by as_solver_set_states_*), and before
         // anything queued there later (as_solver_sync, result and state reads).
-        if (!s->ev_in) AS_CUDA(cudaEventCreateWithFlags(&s->ev_in, cudaEventDisableTiming));
-        if (!s->ev_out) AS_CUDA(cudaEventCreateWithFlags(&s->ev_out, cudaEventDisableTiming));
+        AS_CUDA(ensure_order_events(s));
         AS_CUDA(cudaEventRecord(s->ev_in, s->stream));
         AS_CUDA(cudaStreamWaitEvent(st, s->ev_in, 0));
         int r = record_solve(s, st);

@@ -193,7 +193,9 @@ int32_t as_solver_set_states_f64(as_solver* s, const int32_t* problem_index, int
 int32_t as_solver_set_states_f32(as_solver* s, const int32_t* problem_index, int32_t num_traj,
                                  const float* states);
 /* Same with the states already on the device (in the solver's precision:
- * float for AS_PREC_F32_LOGA, double for AS_PREC_F64), copied device-to-device. */
+ * float for AS_PREC_F32_LOGA, double for AS_PREC_F64), copied device-to-device after
+ * the work queued on `stream` (NULL: the legacy default stream) and before what is
+ * queued there later; with a stream given, the call returns when the copy is done. */
 int32_t as_solver_set_states_device(as_solver* s, const int32_t* problem_index, int32_t num_traj,
                                     const void* states_dev, void* stream);
 

@@ -74,3 +74,52 @@ def test_trajectories_replaced_behind_a_queued_solve():
         r, z = s.results(), s.GetSatStates(np.float32)
         assert np.array_equal(z, want[1])
         assert all(np.array_equal(r[k], want[0][k]) for k in r)
+
+
+@pytest.mark.parametrize("own", [False, True])
+def test_device_states_follow_their_stream(own):
+    """States that work queued on the caller's stream still writes are the ones copied in, and
+    the tensor may be overwritten right after the call."""
+    lits, lens, _ = make_instance("planted", 200, 840, 3, seed=1)
+    p = A.SatProblem.from_arrays(lits, lens)
+    x = torch.from_numpy(initial_states(p.n, p.m, 64, seed=2).astype(np.float32)).cuda()
+    s = A.SatSolver([p], precision=A.AS_PREC_F32_LOGA, device=0)
+    index = np.zeros(64, np.int32)
+    s.SetSatStates(index, x)  # the buffers are there before
+    big = torch.zeros(1 << 28, device="cuda")
+    late = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream() if own else torch.cuda.default_stream()):
+        for _ in range(8):
+            big += 1  # milliseconds of work in front
+        late.copy_(x)
+        s.SetSatStates(index, late)
+        late.zero_()
+    assert np.array_equal(s.GetSatStates(np.float32), x.cpu().numpy().reshape(-1))
+
+
+def test_device_states_set_behind_a_queued_solve():
+    """The states of the next solve do not reach the one that is running."""
+    problems, index, x = uneven()
+    s = A.SatSolver(problems, precision=A.AS_PREC_F32_LOGA, device=0)
+    s.SetEpsilon(1e-6)
+    s.SetMaxTime(1e8)
+    s.SetMaxSteps(30)
+    s.SetBatchSize(30)
+    a = torch.from_numpy(x).cuda()
+    b = a.roll(1).clamp(-0.9, 0.9).abs() + 0.05
+    torch.cuda.synchronize()
+    want = []
+    for y in (a, b):
+        s.SetSatStates(index, y)
+        s.Solve()
+        want.append((s.results(), s.GetSatStates(np.float32)))
+    for stream in (None, torch.cuda.Stream()):
+        s.SetSatStates(index, a, stream=stream)
+        s.SolveAsync()
+        s.SetSatStates(index, b, stream=stream)
+        s.SolveAsync()
+        s.Sync()
+        r, z = s.results(), s.GetSatStates(np.float32)
+        assert np.array_equal(z, want[1][1])
+        assert all(np.array_equal(r[k], want[1][0][k]) for k in r)
