@@ -441,6 +441,7 @@ struct as_problem {
     // Packed on first use of each layout.
     PackedProblem packed_[3];
     bool have_[3] = {false, false, false};
+    long long slots_ = -1;
     std::mutex mu_;
     DevicePool dev[3];        // lazily uploaded for the device primitives
     Workspace work[3];        // scratch of the primitives of instances beyond one SM
@@ -465,6 +466,12 @@ struct as_problem {
         packed_[layout].q = q;
         packed_[layout].b = b;
         return packed_[layout];
+    }
+    // Slots of any of its layouts, without packing one.
+    long long slots() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (slots_ < 0) slots_ = packed_slots(host);
+        return slots_;
     }
     bool standard_model() const { return !tanh && !(b > 0.0); }
     void pack_all() {}
@@ -817,15 +824,18 @@ int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename St
             else return AS_OK;
         }
     }
-    if (p->host.n >= 32768) return AS_OK;  // never compact
-    const auto& q = p->packed(layout);
+    const int n = p->host.n, m = p->host.m;
+    if (n >= 32768) return AS_OK;  // never compact
     int dev = 0, occ = 0;
     DeviceLimits D;
     AS_CUDA(cudaGetDevice(&dev));
     int r = device_limits(dev, &D);
     if (r) return r;
-    const size_t smem = one ? rhs1_smem_bytes(q.n, q.m, q.nslots) : rhs2_smem_bytes(q.n, q.m, q.nslots);
-    if (!q.compact || smem + 1024 > (size_t)D.smem_optin) {
+    // (a layout that does not fit is not packed for nothing)
+    const long long nslots = p->slots();
+    size_t smem = SIZE_MAX / 2;
+    if (nslots <= 65535) smem = one ? rhs1_smem_bytes(n, m, (int)nslots) : rhs2_smem_bytes(n, m, (int)nslots);
+    if (smem + 1024 > (size_t)D.smem_optin) {
         if constexpr (sizeof(V) == 8 && sizeof(T) == 4 && BT == 1024)  // pairs that do not fit
             return launch_rhs_staged<float, LOGA, KMAX, EXACT, BT>(p, x, d, ns, st, done);
         return AS_OK;
@@ -839,7 +849,7 @@ int launch_rhs_staged(as_problem* p, const typename Staged<V>::T* x, typename St
     // bulk stores need dxdt congruent with x mod 16 bytes (same staging offsets)
     const int bulk_out = ((reinterpret_cast<uintptr_t>(x) - reinterpret_cast<uintptr_t>(d)) & 15u) == 0;
     if ((r = ensure_status(p, dev))) return r;
-    fn<<<grid, BT, smem, st>>>(p->dev[layout].host_inst[0], x, d, ns, (long long)(q.n + q.m), bulk_out,
+    fn<<<grid, BT, smem, st>>>(p->dev[layout].host_inst[0], x, d, ns, (long long)n + m, bulk_out,
                                p->rhs_status.as<int>());
     AS_CUDA(cudaGetLastError());
     *done = true;

@@ -795,6 +795,15 @@ bool pack_parts(const HostProblem& p, const PackedProblem& q, int nparts, PartLa
     return true;
 }
 
+long long packed_slots(const HostProblem& p) {
+    std::vector<int32_t> degree(p.n, 0);
+    for (int32_t l : p.storage) degree[std::abs(l) - 1]++;
+    std::sort(degree.begin(), degree.end(), [](int a, int b) { return a > b; });
+    long long rows = 0;  // a slice of 32 variables is as wide as its largest degree, its first
+    for (int v = 0; v < p.n; v += 32) rows += degree[v];
+    return 32 * rows;
+}
+
 PackedProblem pack(const HostProblem& p, int mode) {
     const bool permute_literals = mode != kPackReference;
     PackedProblem q;

@@ -133,5 +133,8 @@ enum PackMode : int {
     kPackF32Pair = 2,    // literals may be reordered; 16-lane bank-pair groups + clause banks
 };
 PackedProblem pack(const HostProblem& p, int mode);
+// The slots of every packing of p (PackedProblem::nslots): they follow from the degrees alone,
+// in microseconds where a packing takes tens of milliseconds.
+long long packed_slots(const HostProblem& p);
 
 }  // namespace asb
