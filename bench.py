@@ -260,6 +260,14 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    from oracle import Reference
+    try:
+        Reference()
+    except (FileNotFoundError, OSError) as e:
+        why = "not built: its sources are not here" if isinstance(e, FileNotFoundError) else f"does not load: {e}"
+        print(json.dumps({"impl": "reference", "unavailable": f"reference CPU solver {why}"}), flush=True)
+        return
     probs, pidx, ics = make_workload(0, args.instances, args.traj)
     units = cpu_sample_units(args.instances, args.traj)
     threads = os.cpu_count() or 1
