@@ -294,7 +294,7 @@ struct Variant {
     int cl;         // CTAs per trajectory (thread-block cluster), global storage only
     SolveFn fn;
     size_t bytes_per_value;
-    bool lean = false;  // solve_kernel_fast: FP32, plain CTDS, offset-carrying literal words
+    bool lean = false;  // solve_kernel_fast: plain CTDS, K = 3 or 4, both precisions
     const char* name() const { return lean ? "solve_kernel_fast" : "solve_kernel"; }
 };
 
@@ -553,7 +553,7 @@ struct as_solver {
     int track_best = 0;
     int forced_bt = 0;
     int forced_cl = 0;     // CTAs per trajectory in global-storage mode (0 = automatic)
-    int kernel_choice = AS_KERNEL_AUTO;  // AS_KERNEL_GENERIC: never the lean FP32 kernel
+    int kernel_choice = AS_KERNEL_AUTO;  // AS_KERNEL_GENERIC: never the lean kernel
     int storage_mode = 0;  // 0 automatic, 1 shared memory, 2 global storage, 3 stream
     std::unique_ptr<StreamPlan> sp;  // streamed solver state
     std::unique_ptr<AdjointPlan> ap; // adjoint buffers
@@ -1022,7 +1022,7 @@ int32_t as_rhs_check(as_problem* p, void* stream) {
     if (dev != on) cudaSetDevice(dev);
     if (e != cudaSuccess) return fail(AS_ERR_CUDA, std::string("as_rhs_check: ") + cudaGetErrorString(e));
     if (word)
-        return fail(AS_ERR_TIMEOUT, "as_rhs_f32: a bulk copy did not complete within 2 s; the states "
+        return fail(AS_ERR_TIMEOUT, "as_rhs: a bulk copy did not complete within 2 s; the states "
                                     "of the affected CTA hold NaN");
     return AS_OK;
 }

@@ -202,7 +202,9 @@ __host__ __device__ inline size_t adjoint_smem_values(int n, int m, int nslots, 
     const size_t Ep = (size_t)((n + m + 3) & ~3), mp = (size_t)((m + 3) & ~3), np = (size_t)((n + 1 + 3) & ~3);
     return (backward ? 12 * Ep + mp + 2 * np : 6 * Ep + np) + (weighted ? mp : 0) + (size_t)nslots + 1;
 }
-// The largest instance an adjoint call takes: fifteen vectors of E values have to fit.
+// The largest instance an adjoint call takes.  The kernels need less (adjoint_smem_values); the
+// limit of fifteen vectors of E values is that of an earlier layout, kept so that the same
+// calls are refused.
 __host__ __device__ inline size_t adjoint_limit_values(int n, int m, int nslots) {
     const size_t Ep = (size_t)((n + m + 3) & ~3);
     return 15 * Ep + 2 * (size_t)((n + 1 + 3) & ~3) + (size_t)nslots + 1;

@@ -384,10 +384,4 @@ __device__ __forceinline__ int group_sum(const Grp<CL>& g, int v, int* red) {
     return s;
 }
 
-// Block max (FP64) whose result is post-processed by thread 0 (single-CTA kernels).
-template <typename F>
-__device__ __forceinline__ double block_max_then(double v, double* red, F&& fn) {
-    return group_max_then<1>(Grp<1>(), v, red, fn);
-}
-
 }  // namespace asb

@@ -704,7 +704,7 @@ bool pack_parts(const HostProblem& p, const PackedProblem& q, int nparts, PartLa
     if (p.n >= 8191 || p.k > 16 || nparts < 1 || (int)q.iperm.size() != p.n) return false;
     const int n = p.n, m = p.m, k = p.k, ns = (n + 31) / 32;
     if (nparts == 1) {
-        // one part is the FP32 packing itself: its clause grouping, literal order and slots
+        // one part is the packing itself: its clause grouping, literal order and slots
         if (q.nslots >= (1 << 17)) return false;
         out.nparts = 1;
         out.max_slots = q.nslots;

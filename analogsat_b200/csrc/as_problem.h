@@ -95,17 +95,20 @@ struct PackedProblem {
     std::vector<int32_t> icperm;   // public -> internal clause
     std::vector<int32_t> deg;      // occurrences of an internal variable
     int max_degree = 0;
-    long bank_wavefronts = 0;      // shared-memory wavefronts of one gather pass (>= 32-clause groups x k)
+    // shared-memory wavefronts of one gather pass over 4-byte spins (>= 32-clause groups x k),
+    // kPackF32Pair: over 8-byte ones (>= 16-clause groups x k)
+    long bank_wavefronts = 0;
     // CTDS variant of the instance (ISat implementation and parameters): tanh = 1 is
     // CpuSatTanh with slope q, b the bias coefficient (ISat::Set_B; 0 = off).
     int tanh = 0;
     double q = 1.1, b = 0.0;
-    // clause parts of the lean FP32 kernel's global-rows form (0: none) and the slots of
+    // clause parts of the lean kernel's parts forms (0: none; FP64 has one) and the slots of
     // the largest part (set by the solver that builds the PartLayout)
     int lean_parts = 0, lean_part_slots = 0;
 };
 
-// Clause parts of the lean FP32 solver's global-rows form: the clauses are split by
+// Clause parts of the lean solver's FP32 global-rows form (and, in one part, of its FP64
+// forms): the clauses are split by
 // public index into `nparts` ranges, each with its own bank-aware warp grouping and
 // its own SELL contribution slots (rows of a variable in public clause order), all
 // parts sharing one shared-memory slot buffer of max_slots + 1 entries.  The variable
@@ -123,7 +126,7 @@ struct PartLayout {
     std::vector<int32_t> icperm;     // public -> internal clause
     std::vector<uint32_t> words;     // [m][k]
 };
-// Builds the parts layout of an instance on the variable order of its FP32 packing q;
+// Builds the parts layout of an instance on the variable order of its packing q;
 // false (layout empty) when N >= 8191 or a part has 2^17 slots or more.
 bool pack_parts(const HostProblem& p, const PackedProblem& q, int nparts, PartLayout& out);
 

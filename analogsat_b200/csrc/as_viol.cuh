@@ -12,10 +12,11 @@
 //                     spread over many CTAs, counts added up with integer atomics
 //                     (order-independent, so still exact and deterministic).
 //
-// Bound by the reads of the spins, 4 N bytes per FP32 state: 16,384 states of N = 1000,
-// M = 4250 took 102 us with one state per CTA pass (every literal word and every spin
-// gathered again for each state), 25 us here (10 us of it the reads at 6.5 TB/s; 33 us with
-// eight loads in flight per thread instead of sixteen).
+// 16,384 states of N = 1000, M = 4250 took 102 us with one state per CTA pass (every literal
+// word and every spin gathered again for each state), 25 us here (33 us with eight loads in
+// flight per thread instead of sixteen).  The spins' reads, 4 N bytes per FP32 state, are
+// 10 us of it at 6.5 TB/s: a CTA's reads and clause checks follow one another, and the
+// CTAs of the one wave are in step, so the two add up.
 #pragma once
 
 #include "as_device.cuh"

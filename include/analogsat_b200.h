@@ -97,8 +97,9 @@ int32_t as_problem_get_clauses(const as_problem* p, int32_t* literals, int32_t* 
 
 /* Device-layout diagnostics of the packing for `precision` (no reference
  * counterpart): contribution slots, largest variable degree, shared-memory
- * wavefronts of one spin-gather pass after bank-aware clause grouping (the ideal is
- * k * ceil(M/32)), and whether the shared-memory kernels accept the instance.
+ * wavefronts of one spin-gather pass over 4-byte spins after bank-aware clause grouping
+ * (the ideal is k * ceil(M/32); the 8-byte spins of FP64 kernels take about twice as
+ * many, served per 16 lanes), and whether the shared-memory kernels accept the instance.
  * `precision` may also be AS_LAYOUT_F32_PAIR, the packing of the FP32 device RHS
  * (as_rhs_f32) that holds two states per shared element; its wavefronts are
  * counted per 16-lane half-warp (ideal k * ceil(M/16)). */
@@ -141,9 +142,9 @@ int32_t as_rhs_f32(as_problem* p, const float* x, float* dxdt, int32_t num_state
 /* FP64 variant, linear a: bit-identical to CpuSat<double>::GetDerivatives. */
 int32_t as_rhs_f64(as_problem* p, const double* x, double* dxdt, int32_t num_states, void* stream);
 /* Device-side status of the earlier asynchronous as_rhs_* calls on p (no reference
- * counterpart; the reference RHS has no waits).  The FP32 RHS moves states through
- * shared memory with asynchronous bulk copies and waits for them at most two
- * seconds; a copy that has not completed by then (a broken device, never a normal
+ * counterpart; the reference RHS has no waits).  For most instances that fit one SM the
+ * RHS of either precision moves states through shared memory with asynchronous bulk
+ * copies and waits for them at most two seconds; a copy that has not completed by then (a broken device, never a normal
  * run) leaves NaN in the outputs of the states that CTA had left and sets a status
  * word of the problem.  as_rhs_check waits for `stream`, reads and clears that word,
  * and returns AS_ERR_TIMEOUT if it was set, else AS_OK. */
@@ -265,8 +266,11 @@ int32_t as_solver_append_perf(as_solver* s, int32_t traj, const char* path, cons
 int32_t as_solver_get_launch_shape(as_solver* s, int32_t* threads, int32_t* ctas, int32_t* smem_bytes,
                                    int32_t* ctas_per_sm);
 /* Force the CTA size (a multiple of 32 in [32, 1024]) of the next solves; 0 restores
- * the automatic choice (the fewest threads that give every thread about the same
- * clause count, at least four).  Used by the autotuner. */
+ * the automatic choice: the fewest threads that give every thread about the same
+ * clause count, at least four; 1,024 where an SM holds one trajectory; and with fewer
+ * trajectories than would fill the GPU the threads that this leaves free, up to one
+ * per clause (not with the bias term, whose rounding follows the CTA size).  Used by
+ * the autotuner. */
 int32_t as_solver_force_threads(as_solver* s, int32_t threads);
 /* Solver kernel of the shared-memory mode (no reference counterpart).  AS_KERNEL_AUTO
  * (default) runs instances with the plain CTDS right-hand side (no tanh variant, no bias
@@ -305,7 +309,8 @@ int32_t as_solver_set_storage_mode(as_solver* s, int32_t mode);
 int32_t as_solver_set_stream_parts(as_solver* s, int32_t parts);
 /* CTAs per trajectory in global-storage mode (no reference counterpart): 0 picks
  * automatically (a thread-block cluster of 4 or 8 CTAs when there are few
- * trajectories, so that they still cover the whole GPU), 1, 4 or 8 force it. */
+ * trajectories, so that they still cover the whole GPU, but one CTA for instances that
+ * the lean kernel takes in one clause part, which is faster so), 1, 4 or 8 force it. */
 int32_t as_solver_set_cluster_size(as_solver* s, int32_t ctas);
 
 /* ---- gradients (no counterpart in the reference: it has no differentiation) --
