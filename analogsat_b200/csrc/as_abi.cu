@@ -961,17 +961,31 @@ int launch_viol(as_problem* p, const T* x, int* c, int ns, cudaStream_t st) {
     const int sms = D.sms;
     if (compact) {  // N < 32768: the masks fit one SM
         const size_t smem = 4 * ((size_t)I.n + 1);
-        // States per group: as many as 32 while every SM still gets about four CTAs (so
-        // that the mask loads of one CTA overlap the clause checks of another), fewer for
-        // few states.  CTAs of a call with no more groups than SMs run alone on their
-        // SM and get all its threads.
-        const int resident = std::max(1, std::min(4, (int)(200 * 1024 / (smem + 1024))));
-        const int per = std::max(1, std::min(32, (ns + sms * resident - 1) / (sms * resident)));
+        // A group's clauses cost the same for one state as for 32, so the states of a call that
+        // 32 to an SM can hold are split over one CTA per SM, all its threads in it (an
+        // instance of no more than 1,024 variables and clauses: 256), a multiple of four to a group
+        // (truth_mask loads four at a time).  us a launch with four CTAs of 256 threads per SM
+        // and fewer states to a group, and so: FP32 N = 5000, M = 21,000, 200 states 28.6 and
+        // 12.5 (one CTA of 256 threads per state, without masks, 16), 1,500 37.4 and 14.5,
+        // 4,736 45.2 and 24.7; N = 1000, M = 4200 8.3, 11.2, 12.4 and 6.3, 8.0, 8.4.  More
+        // states: groups of up to 32 and about four CTAs per SM, so that the mask loads of one
+        // CTA overlap the clause checks of another (N = 1000, 16,384 states 16.6, CTAs of 1,024
+        // threads 25).
+        int per, bt;
+        if (ns <= 32 * sms) {
+            const int share = (ns + sms - 1) / sms;
+            per = share == 1 ? 1 : (share + 3) / 4 * 4;
+            bt = std::max(I.n, I.m) <= 1024 ? 256 : 1024;
+        } else {
+            const int resident = std::max(1, std::min(4, (int)(200 * 1024 / (smem + 1024))));
+            per = std::max(1, std::min(32, (ns + sms * resident - 1) / (sms * resident)));
+            bt = (ns + per - 1) / per > sms ? 256 : 1024;
+        }
         const int grid = (ns + per - 1) / per;
-        auto fn = grid > sms ? &viol_group_kernel<T, KMAX, EXACT, 256> : &viol_group_kernel<T, KMAX, EXACT, 1024>;
+        auto fn = bt == 256 ? &viol_group_kernel<T, KMAX, EXACT, 256> : &viol_group_kernel<T, KMAX, EXACT, 1024>;
         int occ = 0;
-        if (smem > 47 * 1024 && (r = prepare_kernel(p, (const void*)fn, grid > sms ? 256 : 1024, smem, dev, &occ))) return r;
-        fn<<<grid, grid > sms ? 256 : 1024, smem, st>>>(I, x, c, ns, stride, per);
+        if (smem > 47 * 1024 && (r = prepare_kernel(p, (const void*)fn, bt, smem, dev, &occ))) return r;
+        fn<<<grid, bt, smem, st>>>(I, x, c, ns, stride, per);
     } else {
         const int groups = (ns + 31) / 32, gy = std::min(groups, 65535);
         if ((r = p->work[prec].begin(4 * (size_t)groups * ((size_t)I.n + 1), st))) return r;
