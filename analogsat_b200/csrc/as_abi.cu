@@ -1207,6 +1207,44 @@ int plan_units(as_solver* s, const int32_t* problem_index, int num_traj) {
     return AS_OK;
 }
 
+// FP64 instances that one SM holds: the lean kernel's rows are padded to blocks of 32, which
+// can leave room for one CTA fewer per SM than the general kernel's vectors.  Where that
+// costs the call a whole wave of trajectories, the general kernel takes it, with the same
+// results (us, 50 steps: N = 200, M = 840, 1,500 trajectories, two lean CTAs per SM in six waves
+// 3,590, three general ones in four 3,250; N = 150, 1,500 in four and three 2,560 and 2,400;
+// N = 150, 700 in two and two 1,330 and 1,470).  `lean` is the instances' variant, `qs` the
+// instances of its launch, *out the variant to take.
+int fewer_waves(as_solver* s, int lean, const std::vector<const PackedProblem*>& qs, int units, int* out) {
+    const auto& vs = variants();
+    *out = lean;
+    if (!vs[lean].lean || vs[lean].gs || vs[lean].precision != AS_PREC_F64 || s->forced_bt) return AS_OK;
+    int general = -1;
+    for (int i = 0; i < (int)vs.size(); i++)
+        if (!vs[i].lean && !vs[i].gs && vs[i].precision == AS_PREC_F64 && vs[i].exact && vs[i].kmax == vs[lean].kmax)
+            general = i;
+    if (general < 0) return AS_OK;
+    int waves[2] = {0, 0};
+    for (int g = 0; g < 2; g++) {
+        const Variant& v = vs[g ? general : lean];
+        size_t smem = 0;
+        int bt = 64, m = 1, occ = 0;
+        for (const PackedProblem* q : qs) {
+            if (!fits(v, *q, s->precision, s->smem_limit)) return AS_OK;
+            smem = std::max(smem, solver_smem(v, *q));
+            bt = std::max(bt, preferred_bt(*q));
+            m = std::max(m, q->m);
+        }
+        const int r = solver_threads(smem, bt, m, false, units, s->sm_count, s->device, &bt);
+        if (r) return r;
+        AS_CUDA(raise_smem_limit((const void*)v.fn, smem));
+        AS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v.fn, bt, smem));
+        if (occ < 1) return AS_OK;
+        waves[g] = (units + s->sm_count * occ - 1) / (s->sm_count * occ);
+    }
+    if (waves[1] < waves[0]) *out = general;
+    return AS_OK;
+}
+
 // The unit tables, by the solver's own stream: a copy on the default stream is not ordered
 // with the kernels on this one, which does not wait for it.
 int upload_unit_tables(as_solver* s, const std::vector<int>& ui, const std::vector<long long>& us,
@@ -1242,6 +1280,24 @@ int build_groups(as_solver* s) {
         }
         if (pv[p] < 0)
             return fail(AS_ERR_UNSUPPORTED, "no compiled launch shape fits problem " + std::to_string(p));
+    }
+    if (s->precision == AS_PREC_F64) {
+        std::vector<int> per_problem(np, 0);
+        for (int t = 0; t < num_traj; t++) per_problem[s->traj_problem[t]]++;
+        for (int i = 0; i < (int)vs.size(); i++) {
+            std::vector<const PackedProblem*> qs;
+            int units = 0, to = i;
+            for (int p = 0; p < np; p++)
+                if (pv[p] == i && per_problem[p] > 0) {
+                    qs.push_back(&s->problems[p]);
+                    units += per_problem[p];
+                }
+            if (qs.empty() || !vs[i].lean) continue;
+            const int r = fewer_waves(s, i, qs, units, &to);
+            if (r) return r;
+            for (int p = 0; p < np; p++)
+                if (pv[p] == i) pv[p] = to;
+        }
     }
     // global-storage problems with few trajectories: spread each trajectory over a
     // cluster of CTAs so that all trajectories run at once on the whole GPU.  Not those of the
@@ -2290,6 +2346,10 @@ int32_t as_solver_solve_noalloc(as_solver* s, int32_t problem_index, int32_t num
     if (!v)
         return fail(AS_ERR_UNSUPPORTED, "as_solver_solve_noalloc: the instance does not fit one SM's shared "
                                         "memory (only shared-memory launches need no device buffers)");
+    int vi = (int)(v - variants().data());
+    r = fewer_waves(s, vi, {&q}, num_traj, &vi);
+    if (r) return r;
+    v = &variants()[vi];
     const size_t smem = solver_smem(*v, q);
     int bt = s->forced_bt;
     if (!bt) {  // as build_groups does for a call of num_traj trajectories
