@@ -251,7 +251,7 @@ struct DevicePool {
 
 // What the launch rules read of a device, asked of the driver once per device.
 struct DeviceLimits {
-    int sms = 0, smem_optin = 0, smem_per_sm = 0;
+    int sms = 0, smem_optin = 0, smem_per_sm = 0, l2 = 0;
 };
 int device_limits(int dev, DeviceLimits* out) {
     static std::mutex mu;
@@ -266,6 +266,7 @@ int device_limits(int dev, DeviceLimits* out) {
     AS_CUDA(cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev));
     AS_CUDA(cudaDeviceGetAttribute(&L.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     AS_CUDA(cudaDeviceGetAttribute(&L.smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    AS_CUDA(cudaDeviceGetAttribute(&L.l2, cudaDevAttrL2CacheSize, dev));
     known.emplace_back(dev, L);
     *out = L;
     return AS_OK;
@@ -891,6 +892,15 @@ int launch_rhs_rows(as_problem* p, int prec, const T* x, T* d, int ns, cudaStrea
     return r;
 }
 
+// Lanes per row: a 32-byte sector once there are states for most of it.
+template <typename T, bool LOGA, int KMAX, bool EXACT>
+int launch_rhs_lanes(as_problem* p, int prec, const T* x, T* d, int ns, cudaStream_t st) {
+    constexpr int V = 16 / (int)sizeof(T);  // lanes per 16-byte access
+    if (ns == 1) return launch_rhs_rows<T, LOGA, KMAX, EXACT, 1, 1>(p, prec, x, d, ns, st);
+    if (ns <= V) return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 1>(p, prec, x, d, ns, st);
+    return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 2>(p, prec, x, d, ns, st);
+}
+
 template <typename T, bool LOGA, int KMAX, bool EXACT>
 int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
     constexpr int BT = 512;
@@ -914,21 +924,36 @@ int launch_rhs(as_problem* p, const T* x, T* d, int ns, cudaStream_t st) {
         if ((r = prepare_kernel(p, (const void*)fs, BT, smem, dev, &occ))) return r;
         const int grid = std::max(1, std::min(ns, D.sms * std::max(occ, 1)));
         fs<<<grid, BT, smem, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, (T*)nullptr, 0ll);
-    } else if (p->standard_model()) {
-        // Lanes per row: a 32-byte sector once there are states for most of it.
-        constexpr int V = 16 / (int)sizeof(T);  // lanes per 16-byte access
-        if (ns == 1) return launch_rhs_rows<T, LOGA, KMAX, EXACT, 1, 1>(p, prec, x, d, ns, st);
-        if (ns <= V) return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 1>(p, prec, x, d, ns, st);
-        return launch_rhs_rows<T, LOGA, KMAX, EXACT, V, 2>(p, prec, x, d, ns, st);
-    } else {  // tanh variant or bias term: one CTA per state, its vectors in a global slab
+    } else {  // beyond one SM
+        // one CTA per state, its vectors in a global slab: the tanh variant and the bias term
         auto fg = &rhs_batch_kernel<T, LOGA, KMAX, EXACT, BT, true>;
-        if ((r = prepare_kernel(p, (const void*)fg, BT, 0, dev, &occ))) return r;
-        const int grid = std::max(1, std::min(ns, D.sms * std::max(occ, 1)));
         const long long slab_stride = (long long)((vals + 63) / 64 * 64);
-        if ((r = p->work[prec].begin((size_t)grid * slab_stride * sizeof(T), st))) return r;
-        fg<<<grid, BT, 0, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, p->work[prec].buf.template as<T>(),
-                                slab_stride);
-        r = p->work[prec].end(st);
+        bool rows = p->standard_model();
+        if (!rows || q.k > 8) {
+            if ((r = prepare_kernel(p, (const void*)fg, BT, 0, dev, &occ))) return r;
+        }
+        const int grid = std::max(1, std::min(ns, D.sms * std::max(occ, 1)));
+        // ... and FP64 clauses of more than eight literals in batches of eight states an SM or
+        // more, while the slabs in flight fit in L2: the rows' clause kernel, compiled for up to 16
+        // literals in registers, is then bound by issue (us, lengths 3 and 12, rows and so: N = 2500,
+        // M = 3750 300 states 175 and 207, 1,200 645 and 626, 2,400 1,275 and 1,179; N = 3500 2,400
+        // 1,852 and 1,658; N = 5000, beyond L2, 2,764 and 3,191).
+        if (sizeof(T) == 8 && q.k > 8 && ns >= 8 * D.sms && (double)grid * slab_stride * 8.0 <= (double)D.l2) rows = false;
+        if (!rows) {
+            if ((r = p->work[prec].begin((size_t)grid * slab_stride * sizeof(T), st))) return r;
+            fg<<<grid, BT, 0, st>>>(p->dev[prec].host_inst[0], x, d, ns, stride, p->work[prec].buf.template as<T>(),
+                                    slab_stride);
+            r = p->work[prec].end(st);
+        } else {
+            // Rows compiled for lengths up to 4, 8 or 16: with 16 in place of 8 and 4 (145 registers,
+            // 256 predicated products) for all, 2,400 FP64 states of K = 2, N = 3500 took 1,640 us,
+            // 488 so, 1,039 in one CTA per state.
+            if constexpr (!EXACT) {
+                if (q.k <= 4) return launch_rhs_lanes<T, LOGA, 4, false>(p, prec, x, d, ns, st);
+                if (q.k <= 8) return launch_rhs_lanes<T, LOGA, 8, false>(p, prec, x, d, ns, st);
+            }
+            return launch_rhs_lanes<T, LOGA, KMAX, EXACT>(p, prec, x, d, ns, st);
+        }
     }
     AS_CUDA(cudaGetLastError());
     return r;
