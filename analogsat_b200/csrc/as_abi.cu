@@ -496,36 +496,10 @@ struct StreamPlan {
 // one of more than kAdjointKeep bytes is given back after the call, an unsuccessful one too).
 constexpr size_t kAdjointKeep = 1ull << 30;
 struct AdjointPlan {
-    DevBuf ui, us, uw, w, hs, off, ns, used, loss, gx, gw, ck, hsc;
+    DevBuf ui, us, uw, w, hs, off, ns, out, ck, hsc;  // ns: steps, work counters, values asked of the pool; out: grad_x0, grad_w, loss
     std::vector<int> traj;  // the trajectories that ui, us and uw describe
-    // FP32 gradients on their way to the caller's FP64 array.  Pinning costs 2.7 ms for 66 KB,
-    // 5 for 4 MB and 26 to 36 for 64 MB, more than the first call gains: it takes pageable
-    // memory, and a solver called again with as many values pins.
-    float* pinned = nullptr;
-    size_t pinned_values = 0, seen_values = 0;
-    std::vector<float> pageable;
-    ~AdjointPlan() { if (pinned) cudaFreeHost(pinned); }
-    // Room for `values` gradients.
-    float* staging(size_t values) {
-        if (values <= pinned_values) return pinned;
-        if (values <= seen_values) {
-            if (pinned) cudaFreeHost(pinned);
-            pinned = nullptr;
-            pinned_values = 0;
-            if (cudaMallocHost(&pinned, values * sizeof(float)) == cudaSuccess) {
-                pinned_values = values;
-                std::vector<float>().swap(pageable);
-                return pinned;
-            }
-            pinned = nullptr;
-            cudaGetLastError();  // no memory to pin
-        }
-        seen_values = std::max(seen_values, values);
-        if (pageable.size() < values) pageable.resize(values);
-        return pageable.data();
-    }
     void trim() {
-        for (DevBuf* b : {&ck, &hs, &off, &w, &gx, &gw, &hsc})
+        for (DevBuf* b : {&ck, &hs, &off, &w, &out, &hsc})
             if (b->bytes > kAdjointKeep) b->release();
     }
 };
@@ -2466,6 +2440,11 @@ int adjoint_threads(size_t smem, int m, int units, int sms, int smem_per_sm) {
     return std::max(64, std::min(1024, ((m + rounds - 1) / rounds + 31) / 32 * 32));
 }
 
+void touch_pages(void* p, size_t bytes) {
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+}
+
 }  // namespace
 
 int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const double* weights, double* loss,
@@ -2516,11 +2495,10 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     cudaStream_t st = s->stream;
     AS_CUDA(A.hs.alloc(sizeof(double) * (size_t)nt * max_steps));
     AS_CUDA(A.off.alloc(sizeof(long long) * (size_t)nt * ((size_t)max_steps + 1)));
-    AS_CUDA(A.ns.alloc(sizeof(int) * (nt + 2)));
-    AS_CUDA(A.used.alloc(sizeof(unsigned long long)));
-    AS_CUDA(A.loss.alloc(sizeof(double) * nt));
-    AS_CUDA(A.gx.alloc(vb * (size_t)s->total_values));
-    AS_CUDA(A.gw.alloc(sizeof(double) * (size_t)std::max<long long>(wtot, 1)));
+    const size_t used_at = (sizeof(int) * ((size_t)nt + 2) + 7) / 8 * 8, ns_bytes = used_at + sizeof(unsigned long long);
+    AS_CUDA(A.ns.alloc(ns_bytes));
+    const size_t gxn = (size_t)s->total_values, outn = gxn + (size_t)wtot + nt;
+    AS_CUDA(A.out.alloc(sizeof(double) * outn));
     if (A.traj != s->traj_problem) {
         A.traj.clear();
         AS_CUDA(A.ui.alloc(sizeof(int) * nt));
@@ -2551,11 +2529,11 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     P.weights = weights ? A.w.as<double>() : nullptr;
     P.hs = A.hs.as<double>();
     P.nsteps = A.ns.as<int>();
-    P.ckpt_used = A.used.as<unsigned long long>();
+    P.ckpt_used = reinterpret_cast<unsigned long long*>(A.ns.as<char>() + used_at);
     P.ckpt_off = A.off.as<long long>();
-    P.loss = A.loss.as<double>();
-    P.grad_x0 = A.gx.p;
-    P.grad_w = A.gw.as<double>();
+    P.grad_x0 = A.out.as<double>();
+    P.grad_w = P.grad_x0 + gxn;
+    P.loss = P.grad_w + wtot;
     P.num_units = nt;
     P.max_steps = max_steps;
     P.eps = s->eps;
@@ -2575,17 +2553,18 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
         return AS_OK;
     };
     std::vector<int> ns(nt);
+    std::vector<char> counts(ns_bytes);
     while (true) {
         P.ckpt = A.ck.p;
         P.ckpt_cap = (long long)(A.ck.bytes / vb);
-        AS_CUDA(cudaMemsetAsync(A.ns.p, 0, sizeof(int) * (nt + 2), st));
-        AS_CUDA(cudaMemsetAsync(A.used.p, 0, sizeof(unsigned long long), st));
+        AS_CUDA(cudaMemsetAsync(A.ns.p, 0, ns_bytes, st));
         const int r = launch(av->fwd, fvals);
         if (r) return r;
-        unsigned long long used = 0;
-        AS_CUDA(cudaMemcpyAsync(ns.data(), A.ns.p, sizeof(int) * nt, cudaMemcpyDeviceToHost, st));
-        AS_CUDA(cudaMemcpyAsync(&used, A.used.p, sizeof used, cudaMemcpyDeviceToHost, st));
+        AS_CUDA(cudaMemcpyAsync(counts.data(), A.ns.p, ns_bytes, cudaMemcpyDeviceToHost, st));
         AS_CUDA(cudaStreamSynchronize(st));
+        unsigned long long used = 0;
+        std::memcpy(&used, counts.data() + used_at, sizeof used);
+        std::memcpy(ns.data(), counts.data(), sizeof(int) * nt);
         for (int t = 0; t < nt; t++)
             if (ns[t] < 0)
                 return fail(AS_ERR_UNSUPPORTED, ns[t] == -1 ? "adjoint: more than max_steps steps to reach t_end"
@@ -2595,9 +2574,13 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     }
     int r = launch(av->bwd, bvals);
     if (r) return r;
-    // The recorded steps: the columns in use, gathered on the device.  FP32 gradients go
-    // through a staging buffer (16M values at most at a time); pinned, they arrive while the
-    // host still takes in the rest.
+    // The caller's arrays are often fresh pages, which a copy takes in at a quarter of its rate:
+    // touched here, while the kernel runs.  ms a call (before, FP32 gradients through pinned
+    // memory, widened by the host): 1,024 starts of N = 200 4.94 -> 4.72, 4,096 24 -> 16.5, 3,000
+    // of N = 100 10.6 -> 8.5.
+    touch_pages(grad_x0, sizeof(double) * gxn);
+    touch_pages(grad_w, sizeof(double) * (size_t)wtot);
+    // The recorded steps: the columns in use, gathered on the device.
     std::vector<double> hs;
     const int used_steps = *std::max_element(ns.begin(), ns.end());
     const size_t row = sizeof(double) * used_steps;
@@ -2613,26 +2596,11 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
         }
         hs.resize((size_t)nt * used_steps);
     }
-    const size_t gxn = (size_t)s->total_values, chunk = std::min<size_t>(gxn, 1u << 24);
-    float* staged = nullptr;
-    if (vb == 4) {
-        staged = A.staging(chunk);
-        AS_CUDA(cudaMemcpyAsync(staged, A.gx.p, 4 * chunk, cudaMemcpyDeviceToHost, st));
-    } else {
-        AS_CUDA(cudaMemcpyAsync(grad_x0, A.gx.p, 8 * gxn, cudaMemcpyDeviceToHost, st));
-    }
-    AS_CUDA(cudaMemcpyAsync(loss, A.loss.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
-    AS_CUDA(cudaMemcpyAsync(grad_w, A.gw.p, sizeof(double) * wtot, cudaMemcpyDeviceToHost, st));
+    AS_CUDA(cudaMemcpyAsync(grad_x0, P.grad_x0, sizeof(double) * gxn, cudaMemcpyDeviceToHost, st));
+    AS_CUDA(cudaMemcpyAsync(grad_w, P.grad_w, sizeof(double) * wtot, cudaMemcpyDeviceToHost, st));
+    AS_CUDA(cudaMemcpyAsync(loss, P.loss, sizeof(double) * nt, cudaMemcpyDeviceToHost, st));
     if (!hs.empty()) AS_CUDA(cudaMemcpyAsync(hs.data(), A.hsc.p, row * nt, cudaMemcpyDeviceToHost, st));
     AS_CUDA(cudaStreamSynchronize(st));
-    for (size_t o = 0; vb == 4 && o < gxn; o += chunk) {
-        const size_t c = std::min(chunk, gxn - o);
-        if (o > 0) {
-            AS_CUDA(cudaMemcpyAsync(staged, A.gx.as<float>() + o, 4 * c, cudaMemcpyDeviceToHost, st));
-            AS_CUDA(cudaStreamSynchronize(st));
-        }
-        for (size_t i = 0; i < c; i++) grad_x0[o + i] = staged[i];
-    }
     if (nsteps) std::copy(ns.begin(), ns.end(), nsteps);
     if (!hs.empty())
         for (int t = 0; t < nt; t++)

@@ -52,7 +52,7 @@ struct AdjointParams {
     unsigned long long* ckpt_used; // values asked of it (more than ckpt_cap: the pass has to be repeated)
     long long* ckpt_off;           // [unit][max_steps + 1] pool offset of each checkpoint, the last at T
     double* loss;                  // [unit]
-    void* grad_x0;                 // public layout, solver precision
+    double* grad_x0;               // public layout, FP64 as the caller's
     double* grad_w;                // per clause, public order
     int num_units, max_steps;
     double eps, t_end;
@@ -279,9 +279,9 @@ __device__ __forceinline__ void load_public(const DevInstance& I, const T* src, 
 }
 
 template <typename T>
-__device__ __forceinline__ void store_public(const DevInstance& I, const T* src, T* dst) {
-    for (int i = threadIdx.x; i < I.n; i += blockDim.x) dst[i] = src[__ldg(I.iperm + i)];
-    for (int j = threadIdx.x; j < I.m; j += blockDim.x) dst[I.n + j] = src[I.n + __ldg(I.icperm + j)];
+__device__ __forceinline__ void store_public(const DevInstance& I, const T* src, double* dst) {
+    for (int i = threadIdx.x; i < I.n; i += blockDim.x) dst[i] = (double)src[__ldg(I.iperm + i)];
+    for (int j = threadIdx.x; j < I.m; j += blockDim.x) dst[I.n + j] = (double)src[I.n + __ldg(I.icperm + j)];
 }
 
 template <typename T>
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(1024, 1) adj_backward_kernel(AdjointParams P) 
             vjp(std::integral_constant<int, 1>{});
         }
         __syncthreads();
-        store_public<T>(I, A.V(6), reinterpret_cast<T*>(P.grad_x0) + P.unit_state[u]);
+        store_public<T>(I, A.V(6), P.grad_x0 + P.unit_state[u]);
         for (int j = tid; j < I.m; j += nt)
             P.grad_w[P.unit_wofs[u] + j] = (double)A.gw[__ldg(I.icperm + j)];
         __syncthreads();

@@ -31,8 +31,7 @@ def same(a, b):
 
 @pytest.mark.parametrize("precision", [A.AS_PREC_F32_LOGA, A.AS_PREC_F64])
 def test_first_and_later_calls_agree(precision):
-    """The first call of a size, the second (which pins its staging buffer), fewer and more
-    trajectories after that."""
+    """The first call of a size, later ones, fewer and more trajectories after that."""
     s, x = setup(precision, starts=40)
     want = {b: gradients(setup(precision)[0], x[:b]) for b in (1, 7, 40)}
     for b in (7, 7, 7, 1, 40, 7, 40, 40, 1):
