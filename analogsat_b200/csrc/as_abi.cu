@@ -978,7 +978,7 @@ int launch_viol(as_problem* p, const T* x, int* c, int ns, cudaStream_t st) {
         } else {
             const int resident = std::max(1, std::min(4, (int)(200 * 1024 / (smem + 1024))));
             per = std::max(1, std::min(32, (ns + sms * resident - 1) / (sms * resident)));
-            bt = (ns + per - 1) / per > sms ? 256 : 1024;
+            bt = 256;
         }
         const int grid = (ns + per - 1) / per;
         auto fn = bt == 256 ? &viol_group_kernel<T, KMAX, EXACT, 256> : &viol_group_kernel<T, KMAX, EXACT, 1024>;
@@ -1217,6 +1217,7 @@ int fewer_waves(as_solver* s, int lean, const std::vector<const PackedProblem*>&
     const auto& vs = variants();
     *out = lean;
     if (!vs[lean].lean || vs[lean].gs || vs[lean].precision != AS_PREC_F64 || s->forced_bt) return AS_OK;
+    if (units <= s->sm_count) return AS_OK;  // one wave of either
     int general = -1;
     for (int i = 0; i < (int)vs.size(); i++)
         if (!vs[i].lean && !vs[i].gs && vs[i].precision == AS_PREC_F64 && vs[i].exact && vs[i].kmax == vs[lean].kmax)
