@@ -424,8 +424,9 @@ class SatSolver:
                                           loss.ctypes.data_as(C.c_void_p), gx.ctypes.data_as(C.c_void_p),
                                           gw.ctypes.data_as(C.c_void_p), ns.ctypes.data_as(C.c_void_p),
                                           hs.ctypes.data_as(C.c_void_p)))
+        steps = hs[:, : int(ns.max())].copy()  # the columns in use, not the whole table
         return dict(loss=loss, grad_x0=gx, grad_w=gw[:msum], nsteps=ns,
-                    step_sizes=[hs[t, : ns[t]].copy() for t in range(nt)])
+                    step_sizes=[steps[t, :k] for t, k in enumerate(ns.tolist())])
 
     def kernel_name(self) -> str:
         """Solver kernel of the last solve's final launch group."""

@@ -2577,10 +2577,12 @@ int32_t as_solver_adjoint(as_solver* s, double t_end, int32_t max_steps, const d
     if (r) return r;
     // The caller's arrays are often fresh pages, which a copy takes in at a quarter of its rate:
     // touched here, while the kernel runs.  ms a call (before, FP32 gradients through pinned
-    // memory, widened by the host): 1,024 starts of N = 200 4.94 -> 4.72, 4,096 24 -> 16.5, 3,000
-    // of N = 100 10.6 -> 8.5.
+    // memory, widened by the host, no touching): 1,024 starts of N = 200 4.93 -> 4.51, 4,096
+    // 24 -> 16, 3,000 of N = 100 10.6 -> 8.1, FP64 7.4 -> 6.6.
     touch_pages(grad_x0, sizeof(double) * gxn);
     touch_pages(grad_w, sizeof(double) * (size_t)wtot);
+    if (step_sizes)
+        for (int t = 0; t < nt; t++) touch_pages(step_sizes + (size_t)t * max_steps, sizeof(double) * ns[t]);
     // The recorded steps: the columns in use, gathered on the device.
     std::vector<double> hs;
     const int used_steps = *std::max_element(ns.begin(), ns.end());
